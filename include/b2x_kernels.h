@@ -48,7 +48,8 @@ typedef struct {
   const B2xVmProgram* host_post;
 } B2xReduceArgs;
 B2X_API int b2x_reduce_splits(int64_t A, int64_t R, int64_t B);
-/* Kernels one call of b2x_launch_reduce enqueues for this shape: 1, or 2 for a split column reduction (B > 1). */
+/* Kernels one call of b2x_launch_reduce enqueues for this shape: 1, or 2 for a column reduction (B > 1) that splits its
+ * rows beyond what the clusters of its column blocks cover. */
 B2X_API int b2x_reduce_launches(int64_t A, int64_t R, int64_t B);
 B2X_API int b2x_launch_reduce(const B2xVmProgram* host_prologue, const B2xReduceArgs* host_args, b2x_stream_t stream);
 

@@ -4,12 +4,15 @@
 //   B == 1 (row reduction): a group of T threads (a warp or a whole CTA) owns one (row, split) piece, walks it with
 //     128-bit vector loads, folds lanes in registers, then warp shuffles and one shared-memory step.
 //   B  > 1 (column reduction): threads are laid out [ry][bx]; each owns V adjacent columns and strides over R, so a
-//     warp reads one contiguous span per row; the ry partials meet in shared memory.
+//     warp reads one contiguous span per row; the ry partials meet in shared memory, those of a cluster of CTAs that
+//     share the rows in distributed shared memory.
 // Long reductions with few outputs are cut into S splits whose partials land in scratch.  A row reduction folds them in
 // the same launch: every CTA takes a ticket when its partials are written, and the CTA that draws the last ticket folds
-// all of them, in index order, so the result does not depend on which CTA that is.  A column reduction folds them with
-// a second launch.  The final value of each output can be handed to a fused consumer program (its VM_SRC_ACC0), which
+// all of them, in index order, so the result does not depend on which CTA that is.  A column reduction takes splits only
+// where its clusters alone would leave the chip idle, and folds them with a second launch.  The final value of each output can be handed to a fused consumer program (its VM_SRC_ACC0), which
 // then does the stores.  HBM-bound: algorithmic bytes = one read of every operand of the prologue.
+#include <cooperative_groups.h>
+
 #include <cstdio>
 #include <map>
 #include <mutex>
@@ -403,46 +406,149 @@ static int direct_kind(const B2xVmProgram& P, const ReduceKArgs& K, int vec) {
   return 0;
 }
 
-// Column reduction.  blockDim = (BX, RY) with BX * RY = 256; thread (bx, ry) owns V adjacent columns.
-template <int V>
-__global__ void __launch_bounds__(256) k_reduce_cols(const __grid_constant__ B2xVmProgram P, const __grid_constant__ ReduceKArgs K, const __grid_constant__ B2xVmProgram Q, int n_bblocks) {
+// Column reduction.  A cluster of CL CTAs owns 128 or 64 adjacent columns (32 without vectors) of one (outer, split) piece;
+// its rows are dealt to the CTAs and their thread rows in turn, so that at any moment the whole cluster sweeps one band
+// of the tensor.  blockDim = (BX, RY) with BX * RY = 256; thread (bx, ry) owns V adjacent columns.  The thread rows meet
+// in shared memory, the CTAs of the cluster through distributed shared memory, always in the same order.
+// HBM-bound; what decides is how many bytes are in flight, i.e. how many CTAs there are.  [8192, 4096] f32 -> [4096]:
+// 3557 us with one CTA per 2048 columns and row split (8 CTAs, one interpreted row in flight per thread) and a second
+// launch for the four splits; 64 column blocks x 8 CTAs with eight 16-byte loads in flight per thread: 27.0 us (5.0 TB/s) on the device.
+// DIRECT: the prologue is the dense tensor itself, f32 (4) or bf16 (2), and the loop is plain loads and arithmetic
+// (direct_cols); 0: the prologue program.  MC: see red_combine_t.
+template <int V, int DIRECT, int MC>
+__global__ void __launch_bounds__(256) k_reduce_cols(const __grid_constant__ B2xVmProgram P, const __grid_constant__ ReduceKArgs K, const __grid_constant__ B2xVmProgram Q,
+                                                     const char* __restrict__ base, int n_bblocks, int CL) {
+  namespace cg = cooperative_groups;
   __shared__ uint32_t smem[256 * V];
   const int BX = blockDim.x, RY = blockDim.y;
+  const int rank = CL > 1 ? (int)(blockIdx.x % (unsigned)CL) : 0;
   const int64_t n_work = K.A * K.S * (int64_t)n_bblocks;
   uint32_t zero[V];
 #pragma unroll
   for (int j = 0; j < V; j++) zero[j] = 0;
   const uint32_t ident = red_identity(K.monoid, K.cls);
-  for (int64_t w = blockIdx.x; w < n_work; w += gridDim.x) {
+  const int64_t step = (int64_t)RY * CL;
+  for (int64_t w = blockIdx.x / (unsigned)CL; w < n_work; w += gridDim.x / (unsigned)CL) {
     const int bb = (int)(w % n_bblocks);
     const int64_t as = w / n_bblocks;
     const int64_t a = as / K.S, s = as % K.S;
     const int64_t b0 = ((int64_t)bb * BX + threadIdx.x) * V;
-    const int64_t r0 = s * K.chunk, r1 = min(K.R, r0 + K.chunk);
+    const int64_t r1 = min(K.R, (s + 1) * K.chunk);
+    int64_t r = s * K.chunk + (int64_t)rank * RY + threadIdx.y;
     uint32_t tot[V];
 #pragma unroll
     for (int j = 0; j < V; j++) tot[j] = ident;
     if (b0 < K.B) {
-      for (int64_t r = r0 + threadIdx.y; r < r1; r += RY) {
-        uint32_t acc[V];
-        vm_run<V>(P, (uint64_t)((a * K.R + r) * K.B + b0), zero, acc);
+      if constexpr (DIRECT != 0) {
+        constexpr int U = 8;                               // rows in flight per thread
+        constexpr int NB = V * DIRECT;                     // bytes per thread and row
+        constexpr int W = (NB + 3) / 4;
+        const char* p = base + ((a * K.R + r) * K.B + b0) * DIRECT;
+        const int64_t pitch = step * K.B * DIRECT;
+        auto fold = [&](const uint32_t (&raw)[W]) {
 #pragma unroll
-        for (int j = 0; j < V; j++) tot[j] = red_combine(tot[j], acc[j], K.monoid, K.cls);
+          for (int j = 0; j < V; j++) {
+            const uint32_t x = DIRECT == 4 ? raw[j % W] : (V == 1 ? raw[0] << 16 : ((j & 1) ? raw[j / 2] & 0xffff0000u : raw[j / 2] << 16));
+            tot[j] = red_combine_t<MC>(tot[j], x, K.monoid, K.cls);
+          }
+        };
+        for (; r + (U - 1) * step < r1; r += U * step, p += U * pitch) {
+          uint32_t raw[U][W];
+#pragma unroll
+          for (int u = 0; u < U; u++) vm_ld_bytes<NB>(p + u * pitch, raw[u]);
+#pragma unroll
+          for (int u = 0; u < U; u++) fold(raw[u]);
+        }
+        for (; r < r1; r += step, p += pitch) {
+          uint32_t raw[W];
+          vm_ld_bytes<NB>(p, raw);
+          fold(raw);
+        }
+      } else {
+        for (; r < r1; r += step) {
+          uint32_t acc[V];
+          vm_run<V>(P, (uint64_t)((a * K.R + r) * K.B + b0), zero, acc);
+#pragma unroll
+          for (int j = 0; j < V; j++) tot[j] = red_combine_t<MC>(tot[j], acc[j], K.monoid, K.cls);
+        }
       }
     }
-    __syncthreads();
+    __syncthreads();                                       // the previous piece's partials have been read
+    uint32_t* mine = smem + (threadIdx.y * BX + threadIdx.x) * V;
 #pragma unroll
-    for (int j = 0; j < V; j++) smem[(threadIdx.y * BX + threadIdx.x) * V + j] = tot[j];
+    for (int j = 0; j < V; j++) mine[j] = tot[j];
     __syncthreads();
-    if (threadIdx.y == 0 && b0 < K.B) {
-      for (int y = 1; y < RY; y++) {
+    for (int h = RY >> 1; h > 0; h >>= 1) {
+      if ((int)threadIdx.y < h) {
+        const uint32_t* other = smem + ((threadIdx.y + h) * BX + threadIdx.x) * V;
 #pragma unroll
-        for (int j = 0; j < V; j++) tot[j] = red_combine(tot[j], smem[(y * BX + threadIdx.x) * V + j], K.monoid, K.cls);
+        for (int j = 0; j < V; j++) { tot[j] = red_combine_t<MC>(tot[j], other[j], K.monoid, K.cls); mine[j] = tot[j]; }
       }
+      __syncthreads();
+    }
+    if (CL > 1) {
+      cg::cluster_group cluster = cg::this_cluster();
+      cluster.sync();
+      if (rank == 0 && threadIdx.y == 0) {
+        for (int c = 1; c < CL; c++) {
+          const uint32_t* other = cluster.map_shared_rank(smem, c) + threadIdx.x * V;
+#pragma unroll
+          for (int j = 0; j < V; j++) tot[j] = red_combine_t<MC>(tot[j], other[j], K.monoid, K.cls);
+        }
+      }
+      cluster.sync();                                      // the partials may go away (exit, next piece)
+    }
+    if (rank == 0 && threadIdx.y == 0 && b0 < K.B) {
 #pragma unroll
       for (int j = 0; j < V; j++) red_write(K, Q, (a * K.S + s) * K.B + b0 + j, tot[j]);
     }
   }
+}
+
+// Bytes per element (4: f32, 2: bf16) of the dense tensor that a column reduction's prologue merely loads, or 0.
+static int direct_cols(const B2xVmProgram& P, const ReduceKArgs& K) {
+  if (P.n_instr != 1 || P.n_tensors != 1 || P.n_dims != 1 || K.cls != VM_F32) return 0;
+  const B2xVmTensor& T = P.tensors[0];
+  const B2xVmInstr& I = P.code[0];
+  if (I.op != VM_LOAD || I.src_kind != VM_SRC_TENSOR || I.src_idx != 0 || I.tc != VM_F32 || I.rnd != VM_RN_NONE) return 0;
+  if (T.stride[0] != 1 || P.dim[0] != K.A * K.R * K.B) return 0;
+  return T.elem == EL_F32 ? 4 : (T.elem == EL_BF16 ? 2 : 0);
+}
+
+// Clusters of 128 columns that cover at least two waves need no row splits on top (and so no second launch): the eight
+// CTAs of a cluster split the rows already.
+static bool cols_covered_by_clusters(int64_t A, int64_t B) { return A * ((B + 127) / 128) * 8 >= 2 * kNumSms - 40; }
+
+template <int V, int DIRECT, int MC>
+static int launch_cols(const B2xVmProgram& P, const ReduceKArgs& K, const B2xVmProgram& Q, cudaStream_t stream) {
+  const int64_t bvecs = (K.B + V - 1) / V;
+  // 128 columns per CTA, or 64 where 128 would leave less than four CTAs per SM ([8192, 4096] f32: 33.4 us with 128, 27.0 with 64)
+  int bx_max = V == 8 ? 16 : 32;
+  if (DIRECT != 0 && V > 1 && K.A * K.S * ((bvecs + bx_max - 1) / bx_max) * 8 < (int64_t)kNumSms * 4) bx_max /= 2;
+  int bx = 1;
+  while (bx < bx_max && bx < bvecs) bx <<= 1;
+  const int ry = 256 / bx;
+  const int n_bblocks = (int)((bvecs + bx - 1) / bx);
+  const int64_t work = K.A * K.S * (int64_t)n_bblocks;
+  // as many CTAs per cluster as it takes to have four per SM, while each thread still has several rows
+  const int64_t rows = K.chunk < K.R ? K.chunk : K.R;
+  int CL = 1;
+  while (CL < 8 && work * CL < (int64_t)kNumSms * 4 && rows >= (int64_t)ry * CL * 8) CL *= 2;
+  int64_t clusters = work;
+  const int64_t cap = (int64_t)kNumSms * 32;
+  if (clusters > cap) clusters = cap;
+  if (clusters < 1) clusters = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(clusters * CL));
+  cfg.blockDim = dim3((unsigned)bx, (unsigned)ry);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)CL; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
+  const char* base = (const char*)P.tensors[0].ptr;
+  return (int)cudaLaunchKernelEx(&cfg, k_reduce_cols<V, DIRECT, MC>, P, K, Q, base, n_bblocks, CL);
 }
 
 static int launch_one(const B2xVmProgram& P, ReduceKArgs K, const B2xVmProgram& Q, int vec, cudaStream_t stream) {
@@ -490,18 +596,19 @@ static int launch_one(const B2xVmProgram& P, ReduceKArgs K, const B2xVmProgram& 
 #undef B2X_ROWS_MC
 #undef B2X_ROWS
   } else {
-    int64_t bvecs = (K.B + vec - 1) / vec;
-    int bx = 1;
-    while (bx < 256 && bx < bvecs) bx <<= 1;
-    int ry = 256 / bx;
-    int n_bblocks = (int)((bvecs + bx - 1) / bx);
-    int64_t blocks = K.A * K.S * (int64_t)n_bblocks;
-    if (blocks > cap) blocks = cap;
-    if (blocks < 1) blocks = 1;
-    dim3 grid((unsigned)blocks), block(bx, ry);
-    if (vec == 8) k_reduce_cols<8><<<grid, block, 0, stream>>>(P, K, Q, n_bblocks);
-    else if (vec == 4) k_reduce_cols<4><<<grid, block, 0, stream>>>(P, K, Q, n_bblocks);
-    else k_reduce_cols<1><<<grid, block, 0, stream>>>(P, K, Q, n_bblocks);
+    const int mc = red_combine_class(K.monoid, K.cls);
+    const int es = (mc == 1 || mc == 2) && vm_static_enabled() ? direct_cols(P, K) : 0;
+    const int wide = es ? 16 / es : 0;                     // columns per 16-byte load
+    const bool aligned = es && K.B % wide == 0 && ((uintptr_t)P.tensors[0].ptr & 15) == 0;
+    int rc;
+#define B2X_COLS(VV, ES_) (mc == 1 ? launch_cols<VV, ES_, 1>(P, K, Q, stream) : launch_cols<VV, ES_, 2>(P, K, Q, stream))
+    if (es == 4) rc = aligned ? B2X_COLS(4, 4) : B2X_COLS(1, 4);
+    else if (es == 2) rc = aligned ? B2X_COLS(8, 2) : B2X_COLS(1, 2);
+    else if (vec == 8) rc = launch_cols<8, 0, 0>(P, K, Q, stream);
+    else if (vec == 4) rc = launch_cols<4, 0, 0>(P, K, Q, stream);
+    else rc = launch_cols<1, 0, 0>(P, K, Q, stream);
+#undef B2X_COLS
+    if (rc) return rc;
   }
   count_launch();
   return (int)cudaGetLastError();
@@ -551,7 +658,7 @@ extern "C" int b2x_reduce_splits(int64_t A, int64_t R, int64_t B) {
 
 extern "C" int b2x_reduce_launches(int64_t A, int64_t R, int64_t B) {
   if (A <= 0 || B <= 0) return 0;
-  return (b2x_reduce_splits(A, R, B) > 1 && R > 0 && B != 1) ? 2 : 1;
+  return (b2x_reduce_splits(A, R, B) > 1 && R > 0 && B != 1 && !b2x::cols_covered_by_clusters(A, B)) ? 2 : 1;
 }
 
 extern "C" int b2x_launch_reduce(const B2xVmProgram* prologue, const B2xReduceArgs* a, b2x_stream_t stream_) {
@@ -587,7 +694,7 @@ extern "C" int b2x_launch_reduce(const B2xVmProgram* prologue, const B2xReduceAr
   }
   static const B2xVmProgram kNoPost{};
   const B2xVmProgram& Q = a->host_post ? *a->host_post : kNoPost;
-  if (S <= 1 || a->R == 0) {
+  if (S <= 1 || a->R == 0 || (a->B != 1 && cols_covered_by_clusters(a->A, a->B))) {
     K.S = 1; K.chunk = a->R > 0 ? a->R : 1; K.out = a->out;
     return launch_one(*prologue, K, Q, vec, stream);
   }

@@ -1856,8 +1856,7 @@ std::string vm_str(const VmBinding& vm) {
 
 int reduce_splits(int64_t A, int64_t R, int64_t B) { return reduce_splits_impl(A, R, B); }
 int reduce_launches(int64_t A, int64_t R, int64_t B) {
-  if (A <= 0 || B <= 0) return 0;
-  return (reduce_splits_impl(A, R, B) > 1 && R > 0 && B != 1) ? 2 : 1;
+  return b2x_reduce_launches(A, R, B);
 }
 
 std::string Plan::dump() const {
