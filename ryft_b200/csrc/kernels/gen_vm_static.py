@@ -91,10 +91,12 @@ def main():
             key = row["hash"]
             ent = seen.setdefault(key, {"row": row, "roles": set()})
             ent["roles"].add((row["role"], row["bn"]))
-            # a GEMM epilogue is built for both wide tile widths: which one a problem takes depends on its K as well
-            if row["role"] == "gemm_tc" and row["bn"] >= 128:
-                ent["roles"].add((row["role"], 128))
-                ent["roles"].add((row["role"], 256))
+            # a GEMM epilogue is built for every tile width: problems with few tiles take narrower ones than the programs
+            # above do, and an interpreted epilogue costs them more than the product (the six launches of a training step
+            # with 200 tokens, widths 136 and 264: 121 us on the device interpreted, 73 us specialised)
+            if row["role"] == "gemm_tc":
+                for width in (64, 128, 256):
+                    ent["roles"].add((row["role"], width))
     entries = sorted(seen.values(), key=lambda e: (e["row"]["n"], e["row"]["hash"]))
     lines = ["// Specialised fused-elementwise programs.  GENERATED by gen_vm_static.py from the launch plans of the benchmark",
              "// programs; regenerate after changing the planner's code generation.", "#pragma once", "namespace b2x {"]

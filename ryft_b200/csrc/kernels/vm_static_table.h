@@ -194,4 +194,4 @@ __host__ inline int vm_static_lookup(uint64_t h) {
 }  // namespace b2x
 #define B2X_VM_STATIC_ELEMENTWISE(X) X(6) X(7) X(9) X(10) X(11) X(12) X(19)
 #define B2X_VM_STATIC_REDUCE(X) X(1) X(2) X(14)
-#define B2X_VM_STATIC_GEMM(X) X(3, 64) X(3, 128) X(3, 256) X(4, 64) X(4, 128) X(4, 256) X(5, 64) X(5, 128) X(5, 256) X(8, 128) X(8, 256) X(13, 128) X(13, 256) X(15, 128) X(15, 256) X(16, 128) X(16, 256) X(17, 128) X(17, 256) X(18, 128) X(18, 256) X(20, 128) X(20, 256) X(21, 128) X(21, 256) X(22, 128) X(22, 256) X(23, 128) X(23, 256)
+#define B2X_VM_STATIC_GEMM(X) X(3, 64) X(3, 128) X(3, 256) X(4, 64) X(4, 128) X(4, 256) X(5, 64) X(5, 128) X(5, 256) X(8, 64) X(8, 128) X(8, 256) X(13, 64) X(13, 128) X(13, 256) X(15, 64) X(15, 128) X(15, 256) X(16, 64) X(16, 128) X(16, 256) X(17, 64) X(17, 128) X(17, 256) X(18, 64) X(18, 128) X(18, 256) X(20, 64) X(20, 128) X(20, 256) X(21, 64) X(21, 128) X(21, 256) X(22, 64) X(22, 128) X(22, 256) X(23, 64) X(23, 128) X(23, 256)
