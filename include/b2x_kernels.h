@@ -108,6 +108,12 @@ typedef struct {
 } B2xAttentionArgs;
 B2X_API int b2x_launch_attention(const B2xAttentionArgs* host_args, int32_t* status, b2x_stream_t stream);
 
+/* Row softmax out[r][:] = exp(x[r][:] - max) / sum over a dense f32 [rows, n] matrix, the chain of reduce max, subtract,
+ * exponential, reduce add and divide (functional.rs:188-219, exponential.rs, arithmetic.rs), with the quotient stored as
+ * f32, bf16 or f16 (`out_elem`).  Rows of at most B2X_SOFTMAX_MAX_ROW elements. */
+#define B2X_SOFTMAX_MAX_ROW 16384
+B2X_API int b2x_launch_softmax(const void* x, void* out, uint8_t out_elem, int64_t rows, int64_t n, b2x_stream_t stream);
+
 /* Ops over 64-bit element types (i64, ui64, f64; linear_algebra.rs:671-701 and communication.rs:821-841 write the
  * reference's worked examples with i64 tensors).  The fused-elementwise programs above keep values in 32-bit registers,
  * so an op that reads or writes a 64-bit tensor runs as one launch of its own: every operand is addressed through

@@ -11,6 +11,7 @@ static b2x::PlanOptions options_from_environment(int num_replicas) {
   b2x::PlanOptions o;
   o.num_replicas = num_replicas > 0 ? num_replicas : 1;
   if (const char* f = getenv("B2X_FUSED_ATTENTION")) o.allow_fused_attention = strcmp(f, "0") != 0;
+  if (const char* f = getenv("B2X_FUSED_SOFTMAX")) o.allow_fused_softmax = strcmp(f, "0") != 0;
   if (const char* f = getenv("B2X_EPILOGUE_FUSION")) o.allow_epilogue_fusion = strcmp(f, "0") != 0;
   if (const char* g = getenv("B2X_GEMM")) o.allow_tensor_core = strcmp(g, "simt") != 0;
   if (const char* f = getenv("B2X_PRECISE_MATH")) o.precise_math = strcmp(f, "0") != 0;

@@ -172,6 +172,11 @@ PJRT_Error* run_plan(PJRT_LoadedExecutable* le, int local_index, int replica, co
         if (!s.coll_detached) outstanding.push_back(s.coll_id);
         break;
       }
+      case StepKind::SOFTMAX: {
+        int rc = b2x_launch_softmax(bind(s.c_src), bind(s.c_dst), (uint8_t)s.r_out_dtype, s.rA, s.rR, cs);
+        if (rc) return kernel_error(rc, s);
+        break;
+      }
       case StepKind::COPY:
         B2X_CUDA(cudaMemcpyAsync(bind(s.c_dst), bind(s.c_src), (size_t)s.c_bytes, cudaMemcpyDeviceToDevice, cs));
         break;

@@ -869,6 +869,7 @@ static PJRT_Error* build_core(PJRT_Client* client, const std::string& code, cons
     po.precision = co.precision;
     if (const char* g = getenv("B2X_GEMM")) po.allow_tensor_core = strcmp(g, "simt") != 0;
     if (const char* f = getenv("B2X_FUSED_ATTENTION")) po.allow_fused_attention = strcmp(f, "0") != 0;
+    if (const char* f = getenv("B2X_FUSED_SOFTMAX")) po.allow_fused_softmax = strcmp(f, "0") != 0;
     if (const char* f = getenv("B2X_EPILOGUE_FUSION")) po.allow_epilogue_fusion = strcmp(f, "0") != 0;
     if (const char* f = getenv("B2X_PRECISE_MATH")) po.precise_math = strcmp(f, "0") != 0;
     if (co.use_spmd_partitioning && co.num_partitions > 1)
@@ -1344,6 +1345,7 @@ static int step_kernel_launches(const Step& s) {
     case StepKind::REDUCE: return s.wide ? 1 : reduce_launches(s.rA, s.rR, s.rB);
     case StepKind::GEMM: return s.g_split_f32 ? 2 : 1;
     case StepKind::ATTENTION: return 1;
+    case StepKind::SOFTMAX: return 1;
     default: return 0;
   }
 }
@@ -1358,7 +1360,7 @@ static PJRT_Error* Ext_StepTiming(B2X_StepTiming_Args* a) {
     for (auto& s : plan.steps) {
       const char* kind = s.kind == StepKind::GEMM ? (s.g_tensor_core ? "gemm_tc " : "gemm_simt ") : s.kind == StepKind::REDUCE ? "reduce " :
                          s.kind == StepKind::ELEMENTWISE ? "elementwise " : s.kind == StepKind::ATTENTION ? "attention " :
-                         s.kind == StepKind::COPY ? "copy " : s.kind == StepKind::WIDE ? "wide " : "collective ";
+                         s.kind == StepKind::COPY ? "copy " : s.kind == StepKind::WIDE ? "wide " : s.kind == StepKind::SOFTMAX ? "softmax " : "collective ";
       le->step_labels.push_back(std::string(kind) + s.label);
       le->step_flops.push_back(s.flops);
       le->step_bytes.push_back(s.bytes);

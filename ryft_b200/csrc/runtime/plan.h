@@ -21,7 +21,7 @@ struct BufRef {
   bool valid() const { return kind != NONE; }
 };
 
-enum class StepKind : uint8_t { ELEMENTWISE, REDUCE, GEMM, ATTENTION, ALL_REDUCE, ALL_GATHER, COPY, WIDE };
+enum class StepKind : uint8_t { ELEMENTWISE, REDUCE, GEMM, ATTENTION, ALL_REDUCE, ALL_GATHER, COPY, WIDE, SOFTMAX };
 
 struct VmBinding {
   B2xVmProgram prog{};             // tensor pointers are null in the plan; bound at launch
@@ -125,6 +125,7 @@ struct PlanOptions {
   int num_partitions = 1;
   bool allow_tensor_core = true;   // B2X_GEMM=simt turns this off (debugging aid)
   bool allow_fused_attention = true;
+  bool allow_fused_softmax = true;
   bool allow_epilogue_fusion = true;
   int precision = 0;               // Precision::{Default,High,Highest}
   bool precise_math = false;       // B2X_PRECISE_MATH=1: no hardware-approximate tanh/exp/log anywhere (by default they are used

@@ -263,6 +263,15 @@ class Planner {
   void classify();
   struct AttnMatch { const Value* q; const Value* k; const Value* v; float scale; bool causal; };
   std::map<const Op*, AttnMatch> attn_;
+  bool users_are(const Value* v, std::initializer_list<const Op*> ops) const;   // read by these ops only, and not returned
+  static const Op* op_of(const Value* v, OpKind k) { return (v->def && v->def->kind == k) ? v->def : nullptr; }
+  bool splat_f32(const Value* v, float* out) const;
+  const Value* last_dim_bcast(const Value* v) const;   // what `v` broadcasts from [..., S] to [..., S, T] along all leading dims
+  std::map<const Op*, const Value*> softmax_;          // the op whose result a row softmax yields -> its operand
+  std::set<const Op*> softmax_ops_;                    // all ops of the matched row softmaxes
+  bool in_softmax(const Op& op) const { return softmax_ops_.count(&op) != 0; }
+  void match_softmax();
+  void emit_softmax(const Op& op, const Value* x);
   void match_attention();
   void emit_attention(const Op& op, const AttnMatch& m);
   void emit_group_for_root(const Value* v);
@@ -625,28 +634,83 @@ VmBinding Planner::GroupBuilder::finish(int final_node) {
 //   M = reduce max over the last dim; E = exp(S - broadcast(M)); L = reduce add(E); P = E / broadcast(L); [convert];
 //   O = dot_general(P, V) contracting P's last dim with V's key dim.
 // Every intermediate must have no user outside the pattern.
+bool Planner::users_are(const Value* v, std::initializer_list<const Op*> ops) const {
+  for (auto o : m_.outputs) if (o == v) return false;
+  for (auto u : v->users) { bool in = false; for (auto o : ops) if (u == o) in = true; if (!in) return false; }
+  return !v->users.empty();
+}
+bool Planner::splat_f32(const Value* v, float* out) const {
+  if (!v->def) return false;
+  if (v->def->kind == OpKind::CONSTANT && v->def->splat && v->type.dtype == DType::F32) { memcpy(out, v->def->const_data.data(), 4); return true; }
+  if (v->def->kind == OpKind::BROADCAST_IN_DIM && v->def->operands[0]->type.num_elements() == 1) return splat_f32(v->def->operands[0], out);
+  return false;
+}
+const Value* Planner::last_dim_bcast(const Value* v) const {
+  const Op* b = op_of(v, OpKind::BROADCAST_IN_DIM);
+  if (!b) return nullptr;
+  const Value* u = b->operands[0];
+  if (u->type.rank() != v->type.rank() - 1) return nullptr;
+  for (int i = 0; i < u->type.rank(); i++) if (b->dims[i] != i || u->type.dims[i] != v->type.dims[i]) return nullptr;
+  return u;
+}
+
+// Row softmax written out over the last dimension of an f32 value: divide(e, sum(e)) with e = exponential(x - max(x)),
+// optionally narrowed by a convert that is the quotient's only reader.  One pass over memory (softmax.cu) instead of the
+// four that the two reductions and the two elementwise groups take.  The values in between must have no other reader.
+void Planner::match_softmax() {
+  if (!opt_.allow_fused_softmax) return;
+  for (auto& up : m_.ops) {
+    const Op& div = *up;
+    if (div.kind != OpKind::DIVIDE || skip_ops_.count(&div)) continue;
+    const Value* q = div.results[0];
+    const int r = q->type.rank();
+    if (r < 1 || q->type.dtype != DType::F32 || q->type.num_elements() == 0 || q->type.dims[r - 1] > B2X_SOFTMAX_MAX_ROW) continue;
+    const Value* e = div.operands[0];
+    const Value* l = last_dim_bcast(div.operands[1]);
+    if (!l || !users_are(div.operands[1], {&div})) continue;
+    const Op* lred = op_of(l, OpKind::REDUCE);
+    float init = 1.f;
+    if (!lred || lred->monoid != Monoid::ADD || lred->operands[0] != e || lred->dims != std::vector<int64_t>{r - 1} || !users_are(l, {div.operands[1]->def}) ||
+        !splat_f32(lred->operands[1], &init) || init != 0.f) continue;
+    const Op* ex = op_of(e, OpKind::EXP);
+    if (!ex || !users_are(e, {&div, lred})) continue;
+    const Op* sub = op_of(ex->operands[0], OpKind::SUBTRACT);
+    if (!sub || !users_are(ex->operands[0], {ex})) continue;
+    const Value* x = sub->operands[0];
+    const Value* m = last_dim_bcast(sub->operands[1]);
+    if (!m || !users_are(sub->operands[1], {sub})) continue;
+    const Op* mred = op_of(m, OpKind::REDUCE);
+    if (!mred || mred->monoid != Monoid::MAX || mred->operands[0] != x || mred->dims != std::vector<int64_t>{r - 1} || !users_are(m, {sub->operands[1]->def}) ||
+        !splat_f32(mred->operands[1], &init) || !(init == -INFINITY)) continue;
+    for (const Op* c : std::initializer_list<const Op*>{div.operands[1]->def, lred, ex, sub, sub->operands[1]->def, mred}) { skip_ops_.insert(c); softmax_ops_.insert(c); }
+    softmax_ops_.insert(&div);
+    const Op* last = &div;
+    if (q->users.size() == 1 && q->users[0]->kind == OpKind::CONVERT && users_are(q, {q->users[0]})) {
+      const DType dt = q->users[0]->results[0]->type.dtype;
+      if (dt == DType::BF16 || dt == DType::F16) { last = q->users[0]; skip_ops_.insert(&div); softmax_ops_.insert(last); }
+    }
+    softmax_[last] = x;
+  }
+}
+
+void Planner::emit_softmax(const Op& op, const Value* x) {
+  const Value* res = op.results[0];
+  Layout L = layout_of(x);
+  if (!is_row_major(x->type.dims, L.strides)) L.buf = emit_strided_copy(L, x->type.dtype, x->type.dims, "copy:softmax_operand");
+  Step s;
+  s.kind = StepKind::SOFTMAX;
+  s.label = "softmax:%" + res->name;
+  s.rR = x->type.dims.back();
+  s.rA = x->type.num_elements() / s.rR;
+  s.c_src = L.buf;
+  s.c_dst = materialise(res);
+  s.r_out_dtype = res->type.dtype;
+  s.bytes = (double)x->type.byte_size() + (double)res->type.byte_size();
+  plan_.steps.push_back(std::move(s));
+}
+
 void Planner::match_attention() {
   if (!opt_.allow_fused_attention) return;
-  auto users_are = [&](const Value* v, std::initializer_list<const Op*> ops) {
-    for (auto o : m_.outputs) if (o == v) return false;
-    for (auto u : v->users) { bool in = false; for (auto o : ops) if (u == o) in = true; if (!in) return false; }
-    return !v->users.empty();
-  };
-  auto op_of = [&](const Value* v, OpKind k) -> const Op* { return (v->def && v->def->kind == k) ? v->def : nullptr; };
-  std::function<bool(const Value*, float*)> splat_f32 = [&](const Value* v, float* out) -> bool {
-    if (!v->def) return false;
-    if (v->def->kind == OpKind::CONSTANT && v->def->splat && v->type.dtype == DType::F32) { memcpy(out, v->def->const_data.data(), 4); return true; }
-    if (v->def->kind == OpKind::BROADCAST_IN_DIM && v->def->operands[0]->type.num_elements() == 1) return splat_f32(v->def->operands[0], out);
-    return false;
-  };
-  auto last_dim_bcast = [&](const Value* v) -> const Value* {   // broadcast of [..., S] to [..., S, T] along all leading dims
-    const Op* b = op_of(v, OpKind::BROADCAST_IN_DIM);
-    if (!b) return nullptr;
-    const Value* u = b->operands[0];
-    if (u->type.rank() != v->type.rank() - 1) return nullptr;
-    for (int i = 0; i < u->type.rank(); i++) if (b->dims[i] != i || u->type.dims[i] != v->type.dims[i]) return nullptr;
-    return u;
-  };
   for (auto& up : m_.ops) {
     const Op& d2 = *up;
     if (d2.kind != OpKind::DOT_GENERAL) continue;
@@ -764,7 +828,7 @@ void Planner::classify() {
   // forward: fusible / cheap
   for (auto& up : m_.ops) {
     const Op& op = *up;
-    if (!is_fusible_kind(op)) continue;
+    if (!is_fusible_kind(op) || in_softmax(op)) continue;
     for (auto r : op.results) {
       ValueState& s = st(r);
       s.fusible = true;
@@ -790,6 +854,11 @@ void Planner::classify() {
   for (int i = (int)m_.ops.size() - 1; i >= 0; i--) {
     const Op& op = *m_.ops[i];
     if (op.kind == OpKind::RETURN) { for (auto v : op.operands) sink(v); continue; }
+    if (in_softmax(op)) {     // a kernel of its own, which reads the row softmax's operand from memory
+      auto it = softmax_.find(&op);
+      if (it != softmax_.end()) sink(it->second);
+      continue;
+    }
     if (is_fusible_kind(op)) {
       const Value* v = op.results[0];
       ValueState& s = st(v);
@@ -1277,7 +1346,7 @@ bool collapse(const std::vector<int64_t>& dims, const std::vector<int64_t>& stri
 // the kernel runs and that reach `res` with unchanged coordinates.  Returns whether `res` itself must still be stored.
 bool Planner::collect_consumer_roots(const Op& op, const Value* res, std::vector<const Value*>* fused_roots) {
   bool res_needs_memory = false;
-  for (auto u : res->users) if (!is_fusible_kind(*u) && !(u->kind == OpKind::REDUCE && u->operands[0] == res)) res_needs_memory = true;
+  for (auto u : res->users) if (in_softmax(*u) || (!is_fusible_kind(*u) && !(u->kind == OpKind::REDUCE && u->operands[0] == res))) res_needs_memory = true;
   for (auto o : m_.outputs) if (o == res) res_needs_memory = true;
   const int my_index = op_index_[&op];
   for (int g : st(res).groups) {
@@ -1590,7 +1659,7 @@ static void step_bufs(const Step& s, std::vector<BufRef>* reads, std::vector<Buf
     case StepKind::ALL_REDUCE: case StepKind::ALL_GATHER:
       for (auto& c : s.colls) { reads->push_back(c.src); writes->push_back(c.dst); }
       break;
-    case StepKind::COPY: reads->push_back(s.c_src); writes->push_back(s.c_dst); break;
+    case StepKind::COPY: case StepKind::SOFTMAX: reads->push_back(s.c_src); writes->push_back(s.c_dst); break;
   }
 }
 
@@ -1749,6 +1818,7 @@ Plan Planner::run() {
     plan_.arg_types.push_back(a->type);
   }
   match_attention();
+  match_softmax();
   classify();
   for (auto a : m_.args) {
     BufRef b;
@@ -1759,6 +1829,7 @@ Plan Planner::run() {
   for (auto& up : m_.ops) {
     const Op& op = *up;
     if (skip_ops_.count(&op)) continue;
+    if (auto it = softmax_.find(&op); it != softmax_.end()) { emit_softmax(op, it->second); continue; }
     switch (op.kind) {
       case OpKind::RETURN: break;
       case OpKind::CONSTANT:
@@ -1899,6 +1970,9 @@ std::string Plan::dump() const {
         o << "]";
         for (int k = 0; k < s.w_n_in; k++) o << " " << buf_str(s.w_in[k]) << ":" << dtype_name(s.w_in_dtype[k]);
         o << " -> " << buf_str(s.w_out) << ":" << dtype_name(s.w_out_dtype) << "\n";
+        break;
+      case StepKind::SOFTMAX:
+        o << "softmax " << s.label << " [" << s.rA << "," << s.rR << "] " << buf_str(s.c_src) << " -> " << buf_str(s.c_dst) << ":" << dtype_name(s.r_out_dtype) << "\n";
         break;
       case StepKind::COPY: o << "copy " << s.label << " " << buf_str(s.c_src) << " -> " << buf_str(s.c_dst) << " " << s.c_bytes << " B\n"; break;
     }
