@@ -28,7 +28,7 @@ __device__ __forceinline__ uint32_t vm_narrow(uint32_t v, uint8_t rnd) {
   }
 }
 
-__device__ __forceinline__ int vm_elem_size(uint8_t e) {
+__host__ __device__ __forceinline__ int vm_elem_size(uint8_t e) {
   switch (e) {
     case EL_PRED: case EL_S8: case EL_U8: return 1;
     case EL_S16: case EL_U16: case EL_F16: case EL_BF16: return 2;

@@ -64,3 +64,37 @@ def test_row_softmax(client, shape, out_dtype):
 def test_row_softmax_of_a_value_that_is_also_returned(client):
     shape = (6, 200)
     check_program(client, softmax_program(shape, extra=True), [np.random.default_rng(4).standard_normal(shape, dtype=np.float32)], "softmax, operand returned", f32_tol=1e-6)
+
+
+# CUDA-core products: one tile, K cut over 2, 4 and 8 CTAs, 64- and 128-row tiles with ragged edges, all four operand forms
+@pytest.mark.parametrize("B,M,K,N", [(1, 2, 3, 2), (1, 1, 2049, 1), (1, 65, 127, 63), (1, 8, 2048, 9), (1, 130, 300, 129), (1, 700, 131, 701), (1, 1290, 129, 1283), (3, 70, 515, 33),
+                                     (1030, 3, 5, 7)])
+@pytest.mark.parametrize("dtype,lc,rc", [("f32", 1, 0), ("bf16", 0, 1), ("f16", 1, 1), ("f32", 0, 0), ("i32", 1, 0), ("i8", 0, 1)])
+def test_cuda_core_product(client, B, M, K, N, dtype, lc, rc):
+    import ryft_b200
+    ls, rs = ([B, M, K] if lc else [B, K, M]), ([B, N, K] if rc else [B, K, N])
+    b = Builder()
+    x = b.arg(ls, dtype); y = b.arg(rs, dtype)
+    text = b.build(b.dot_general(x, y, ([0], [0]), ([2 if lc else 1], [2 if rc else 1]), out_dtype="f32" if dtype in ("f32", "bf16", "f16") else "i32"))
+    assert " simt" in ryft_b200.plan_dump(text)
+    r = np.random.default_rng(9)
+    npdt = configs.np_dtype(dtype)
+    ins = [r.integers(-100, 100, size=s).astype(npdt) if dtype[0] == "i" else r.standard_normal(s, dtype=np.float32).astype(npdt) for s in (ls, rs)]
+    # products of 16-bit values are exact in f32 and an f32 product rounds with 2^-24; K <= 2049 sums do so as well, with random signs
+    check_program(client, text, ins, f"{dtype} {B}x{M}x{K}x{N}", f32_tol=1e-6)
+
+
+# the same kernel's fused epilogues, four columns and one column per run of the program
+@pytest.mark.parametrize("M,K,N", [(100, 520, 136), (77, 640, 61), (1501, 40, 1203)])
+def test_cuda_core_product_with_epilogue(client, M, K, N):
+    import ryft_b200
+    b = Builder()
+    x = b.arg([M, K], "bf16"); y = b.arg([K, N], "bf16"); bias = b.arg([N], "f32")
+    d = b.dot_general(x, y, ([], []), ([1], [0]), out_dtype="f32")
+    s = b.add(d, b.broadcast_in_dim(bias, [1], [M, N]))
+    text = b.build(b.tanh(s), b.convert(s, "bf16"))
+    if " simt" not in ryft_b200.plan_dump(text):
+        pytest.skip("the tensor cores take this product")
+    r = np.random.default_rng(10)
+    ins = [(r.standard_normal(s, dtype=np.float32) * np.float32(0.2)).astype(BF16) for s in ((M, K), (K, N))] + [r.standard_normal((N,), dtype=np.float32)]
+    check_program(client, text, ins, f"epilogue {M}x{K}x{N}", f32_tol=1e-6)
