@@ -36,6 +36,37 @@ PJRT_Error* cuda_error(cudaError_t e, const char* what);
   } while (0)
 }  // namespace b2x
 
+namespace b2x {
+// A point in a stream's work: an event recorded once and never again, shared by everything that has to know when the
+// stream has got there (the outputs of an execution, the views it read, its completion).  One event per execution instead
+// of one per output, argument and completion: creating, recording and destroying them was a third of the execute call.
+struct StreamMark {
+  cudaEvent_t ev = nullptr;
+  cudaStream_t stream = nullptr;
+  ~StreamMark() { if (ev) cudaEventDestroy(ev); }
+};
+using MarkRef = std::shared_ptr<StreamMark>;
+// Records a mark behind the work that `stream` holds now (the stream's device must be current).  The mark exists also when
+// recording failed: whoever waits for it is then told.
+inline cudaError_t mark_stream(cudaStream_t stream, MarkRef* out) {
+  MarkRef m = std::make_shared<StreamMark>();
+  m->stream = stream;
+  cudaError_t e = cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(m->ev, stream);
+  *out = std::move(m);
+  return e;
+}
+// Makes `stream` wait for a mark; nothing to do when the mark lies on the stream itself.
+inline cudaError_t wait_mark(cudaStream_t stream, const MarkRef& m) {
+  return m && m->stream != stream ? cudaStreamWaitEvent(stream, m->ev, 0) : cudaSuccess;
+}
+// Remembers a reader.  A later mark of the same stream covers the earlier one, so the list holds one per stream.
+inline void add_mark(std::vector<MarkRef>* marks, MarkRef m) {
+  for (auto& o : *marks) if (o->stream == m->stream) { o = std::move(m); return; }
+  marks->push_back(std::move(m));
+}
+}  // namespace b2x
+
 // Host-visible completion object.  Thread-safe; callbacks run exactly once, on the thread that completes the event
 // or immediately on the registering thread if it is already complete (reference expectations:
 // crates/ryft-pjrt/src/events.rs:89-144, tests :566-648).
@@ -125,11 +156,11 @@ struct PJRT_Buffer {
   bool from_host = false;     // created by a host-to-device upload: its block is recycled for the next upload of that size
   bool deleted = false;
   std::function<void()> on_delete;
-  cudaEvent_t ready = nullptr;      // recorded on the producing stream
+  b2x::MarkRef ready;               // on the producing stream
   PJRT_Event* definition_error = nullptr;  // set for error buffers
   PJRT_Error_Code err_code = PJRT_Error_Code_OK;
   std::string err_msg;
-  std::vector<cudaEvent_t> pending_reads;  // D2H copies still in flight on the d2h stream
+  std::vector<b2x::MarkRef> pending_reads;  // readers that freeing the memory has to wait for: copies, and executions for views
   std::mutex mu;
   std::atomic<int> ext_refs{0};
   std::vector<int64_t> minor_to_major;
@@ -209,7 +240,7 @@ struct PJRT_Client {
   PJRT_KeyValueGetCallback kv_get = nullptr; void* kv_get_arg = nullptr;
   PJRT_KeyValuePutCallback kv_put = nullptr; void* kv_put_arg = nullptr;
   // completion poller: turns cudaEvents into PJRT_Events off the caller's thread
-  struct Pending { cudaEvent_t ev; int ordinal; PJRT_Event* event; std::function<void(PJRT_Error_Code*, std::string*)> finish; };
+  struct Pending { b2x::MarkRef mark; int ordinal; PJRT_Event* event; std::function<void(PJRT_Error_Code*, std::string*)> finish; };
   std::mutex q_mu;
   std::condition_variable q_cv;
   std::deque<Pending> queue;

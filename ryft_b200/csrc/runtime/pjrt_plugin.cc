@@ -91,11 +91,11 @@ static void poller_main(PJRT_Client* c) {
     }
     PJRT_Error_Code code = PJRT_Error_Code_OK;
     std::string msg;
-    if (p.ev) {
+    if (p.mark) {
       cudaSetDevice(p.ordinal);
-      cudaError_t e = cudaEventSynchronize(p.ev);
+      cudaError_t e = cudaEventSynchronize(p.mark->ev);
       if (e != cudaSuccess) { code = PJRT_Error_Code_INTERNAL; msg = std::string("device work failed: ") + cudaGetErrorString(e); }
-      cudaEventDestroy(p.ev);
+      p.mark.reset();
     }
     if (p.finish) p.finish(&code, &msg);
     if (p.event) { p.event->set(code, msg); p.event->unref(); }
@@ -194,9 +194,9 @@ static void release_buffer_memory(PJRT_Buffer* b) {
   if (b->owns) {
     await_definition(b);
     // every use of the memory was enqueued on the compute stream, or on a transfer stream with a recorded event
-    for (auto ev : b->pending_reads) { cudaStreamWaitEvent(d->compute, ev, 0); cudaEventDestroy(ev); }
+    for (auto& m : b->pending_reads) wait_mark(d->compute, m);
     b->pending_reads.clear();
-    if (b->ready) cudaStreamWaitEvent(d->compute, b->ready, 0);
+    wait_mark(d->compute, b->ready);
     bool kept = false;
     if (b->from_host && b->bytes >= PJRT_Device::kMinRecycledBytes) {
       std::lock_guard<std::mutex> lk(d->recycle_mu);
@@ -215,7 +215,7 @@ static void release_buffer_memory(PJRT_Buffer* b) {
     if (!kept) cudaFreeAsync(b->ptr, d->compute);
     d->bytes_in_use -= (int64_t)b->bytes;
   } else {
-    for (auto ev : b->pending_reads) { cudaEventSynchronize(ev); cudaEventDestroy(ev); }
+    for (auto& m : b->pending_reads) cudaEventSynchronize(m->ev);
     b->pending_reads.clear();
     if (b->on_delete) { cudaStreamSynchronize(d->compute); b->on_delete(); }
   }
@@ -603,8 +603,7 @@ static PJRT_Error* Client_BufferFromHostBuffer(PJRT_Client_BufferFromHostBuffer_
   }
   cudaError_t e = cudaSuccess;
   if (b->bytes) e = cudaMemcpyAsync(b->ptr, src, b->bytes, cudaMemcpyHostToDevice, dev->h2d);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventRecord(b->ready, dev->h2d);
+  if (e == cudaSuccess) e = mark_stream(dev->h2d, &b->ready);
   if (e != cudaSuccess) { release_buffer_memory(b); delete b; return cuda_error(e, "host to device copy"); }
   PJRT_Event* done = new PJRT_Event();
   const bool must_finish_now = a->host_buffer_semantics == PJRT_HostBufferSemantics_kImmutableOnlyDuringCall || !dense;
@@ -616,10 +615,7 @@ static PJRT_Error* Client_BufferFromHostBuffer(PJRT_Client_BufferFromHostBuffer_
     if (pinned || !dense) cudaStreamSynchronize(dev->h2d);
     done->set(PJRT_Error_Code_OK, "");
   } else {
-    cudaEvent_t ev;
-    cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    cudaEventRecord(ev, dev->h2d);
-    a->client->post({ev, dev->cuda_ordinal, done, nullptr});
+    a->client->post({b->ready, dev->cuda_ordinal, done, nullptr});
   }
   a->done_with_host_buffer = done;
   a->buffer = b;
@@ -661,8 +657,7 @@ static PJRT_Error* Client_CreateViewOfDeviceBuffer(PJRT_Client_CreateViewOfDevic
   }
   if (a->stream) {  // work already queued on the producer's stream must finish before this buffer is read
     cudaSetDevice(dev->cuda_ordinal);
-    cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming);
-    cudaEventRecord(b->ready, (cudaStream_t)a->stream);
+    mark_stream((cudaStream_t)a->stream, &b->ready);
   }
   a->buffer = b;
   return nullptr;
@@ -690,7 +685,6 @@ static PJRT_Error* Buffer_Destroy(PJRT_Buffer_Destroy_Args* a) {
   {
     std::lock_guard<std::mutex> lk(a->buffer->mu);
     release_buffer_memory(a->buffer);
-    if (a->buffer->ready) { cudaEventDestroy(a->buffer->ready); a->buffer->ready = nullptr; }
   }
   delete a->buffer;
   return nullptr;
@@ -741,13 +735,7 @@ static PJRT_Error* Buffer_ReadyEvent(PJRT_Buffer_ReadyEvent_Args* a) {
   if (b->err_code != PJRT_Error_Code_OK) { ev->set(b->err_code, b->err_msg); a->event = ev; return nullptr; }
   if (b->deleted) { delete ev; return make_error(PJRT_Error_Code_INVALID_ARGUMENT, "the buffer has been deleted"); }
   if (!b->ready) { ev->set(PJRT_Error_Code_OK, ""); a->event = ev; return nullptr; }
-  // wait for the definition event on a side stream so that later re-records do not matter
-  cudaSetDevice(b->device->cuda_ordinal);
-  cudaEvent_t e2;
-  cudaEventCreateWithFlags(&e2, cudaEventDisableTiming);
-  cudaStreamWaitEvent(b->device->d2h, b->ready, 0);
-  cudaEventRecord(e2, b->device->d2h);
-  b->client->post({e2, b->device->cuda_ordinal, ev, nullptr});
+  b->client->post({b->ready, b->device->cuda_ordinal, ev, nullptr});
   a->event = ev;
   return nullptr;
 }
@@ -756,7 +744,7 @@ static PJRT_Error* copy_to_host(PJRT_Buffer* b, void* dst, size_t offset, size_t
   await_definition(b);
   PJRT_Device* d = b->device;
   B2X_CUDA(cudaSetDevice(d->cuda_ordinal));
-  if (b->ready) B2X_CUDA(cudaStreamWaitEvent(d->d2h, b->ready, 0));
+  B2X_CUDA(wait_mark(d->d2h, b->ready));
   // Small reads (a loss, a metric) go through a pinned staging block and reach `dst` on the poller thread when the copy
   // has finished: the call returns at once even though `dst` is ordinary pageable memory, so a training loop can
   // enqueue its next step before the current one is done.  Larger reads are dominated by the transfer itself.
@@ -769,19 +757,12 @@ static PJRT_Error* copy_to_host(PJRT_Buffer* b, void* dst, size_t offset, size_t
     if (cudaHostAlloc(&staging, PJRT_Device::kStagingBlock, cudaHostAllocDefault) != cudaSuccess) { cudaGetLastError(); staging = nullptr; }
   }
   if (size) B2X_CUDA(cudaMemcpyAsync(staging ? staging : dst, (const char*)b->ptr + offset, size, cudaMemcpyDeviceToHost, d->d2h));
-  cudaEvent_t ev, keep;
-  B2X_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-  B2X_CUDA(cudaEventRecord(ev, d->d2h));
-  B2X_CUDA(cudaEventCreateWithFlags(&keep, cudaEventDisableTiming));
-  B2X_CUDA(cudaEventRecord(keep, d->d2h));
-  // drop read markers that have completed, then remember this one so that freeing the buffer waits for the copy
-  for (auto it = b->pending_reads.begin(); it != b->pending_reads.end();) {
-    if (cudaEventQuery(*it) == cudaSuccess) { cudaEventDestroy(*it); it = b->pending_reads.erase(it); } else ++it;
-  }
-  b->pending_reads.push_back(keep);
+  MarkRef copied;
+  B2X_CUDA(mark_stream(d->d2h, &copied));
+  add_mark(&b->pending_reads, copied);   // freeing the buffer waits for the copy
   PJRT_Event* pe = new PJRT_Event();
   PJRT_Device* dev = d;
-  b->client->post({ev, d->cuda_ordinal, pe, [dev, staging, dst, size](PJRT_Error_Code* code, std::string* msg) {
+  b->client->post({copied, d->cuda_ordinal, pe, [dev, staging, dst, size](PJRT_Error_Code* code, std::string* msg) {
                      if (staging) {
                        if (*code == PJRT_Error_Code_OK) memcpy(dst, staging, size);
                        std::lock_guard<std::mutex> sl(dev->staging_mu);
@@ -819,20 +800,16 @@ static PJRT_Error* copy_to_device_impl(PJRT_Buffer* b, PJRT_Device* dst_dev, PJR
   PJRT_Buffer* nb;
   B2X_RETURN_IF_ERROR(alloc_buffer(dst_dev, b->type, dst_dev->compute, &nb));
   cudaSetDevice(dst_dev->cuda_ordinal);
-  if (b->ready) cudaStreamWaitEvent(dst_dev->compute, b->ready, 0);
+  wait_mark(dst_dev->compute, b->ready);
   cudaError_t e = cudaSuccess;
   if (b->bytes) {
     if (dst_dev == b->device) e = cudaMemcpyAsync(nb->ptr, b->ptr, b->bytes, cudaMemcpyDeviceToDevice, dst_dev->compute);
     else e = cudaMemcpyPeerAsync(nb->ptr, dst_dev->cuda_ordinal, b->ptr, b->device->cuda_ordinal, b->bytes, dst_dev->compute);
   }
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&nb->ready, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventRecord(nb->ready, dst_dev->compute);
+  if (e == cudaSuccess) e = mark_stream(dst_dev->compute, &nb->ready);
   if (e != cudaSuccess) { release_buffer_memory(nb); delete nb; return cuda_error(e, "device to device copy"); }
   // the source must outlive the copy: remember the read on the source buffer
-  cudaEvent_t keep;
-  cudaEventCreateWithFlags(&keep, cudaEventDisableTiming);
-  cudaEventRecord(keep, dst_dev->compute);
-  b->pending_reads.push_back(keep);
+  add_mark(&b->pending_reads, nb->ready);
   *out = nb;
   return nullptr;
 }
@@ -1181,7 +1158,7 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
     for (size_t i = 0; i < n_args; i++) {
       PJRT_Buffer* b = a->argument_lists[k][i];
       await_definition(b);
-      if (b->ready) cudaStreamWaitEvent(dev->compute, b->ready, 0);
+      wait_mark(dev->compute, b->ready);
       L.args.push_back(b->ptr);
     }
     for (size_t o = 0; o < n_outs; o++) {
@@ -1254,6 +1231,12 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
       cudaEventDestroy(join);
       done_stream = dev->comm;
     }
+    // everything this execution has enqueued: on the compute stream, and behind its detached collectives
+    MarkRef computed, done;
+    if (!failed) {
+      mark_stream(dev->compute, &computed);
+      if (done_stream == dev->compute) done = computed; else mark_stream(done_stream, &done);
+    }
     for (size_t o = 0; o < n_outs; o++) {
       PJRT_Buffer* ob = o < L.out_bufs.size() ? L.out_bufs[o] : nullptr;
       if (!ob) {
@@ -1266,8 +1249,7 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
         // an output that no detached collective writes is final when the compute stream gets here (a loss can be read back
         // while the gradients' all-reduce is still running behind the next step)
         const bool on_comm = done_stream != dev->compute && (o >= plan0.out_in_detached.size() || plan0.out_in_detached[o]);
-        cudaEventCreateWithFlags(&ob->ready, cudaEventDisableTiming);
-        cudaEventRecord(ob->ready, on_comm ? done_stream : dev->compute);
+        ob->ready = on_comm ? done : computed;
       }
       if (a->output_lists && a->output_lists[k]) a->output_lists[k][o] = ob;
     }
@@ -1281,17 +1263,8 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
         PJRT_Buffer* b = a->argument_lists[k][i];
         const bool comm_readers = done_stream != dev->compute && (i >= plan0.arg_in_detached.size() || plan0.arg_in_detached[i]);
         if (!b->owns || comm_readers) {
-          cudaEvent_t keep;
-          cudaEventCreateWithFlags(&keep, cudaEventDisableTiming);
-          cudaEventRecord(keep, comm_readers ? done_stream : dev->compute);
           std::lock_guard<std::mutex> bl(b->mu);
-          // a buffer that is an argument step after step would otherwise collect one event per execution
-          size_t kept = 0;
-          for (auto ev : b->pending_reads) {
-            if (cudaEventQuery(ev) == cudaSuccess) cudaEventDestroy(ev); else b->pending_reads[kept++] = ev;
-          }
-          b->pending_reads.resize(kept);
-          b->pending_reads.push_back(keep);
+          add_mark(&b->pending_reads, comm_readers ? done : computed);
         }
       }
     }
@@ -1299,11 +1272,8 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
       PJRT_Event* ev = new PJRT_Event();
       if (failed) ev->set(L.err->code, L.err->message);
       else {
-        cudaEvent_t ce;
-        cudaEventCreateWithFlags(&ce, cudaEventDisableTiming);
-        cudaEventRecord(ce, done_stream);
         PJRT_Device* d = dev;
-        le->client->post({ce, dev->cuda_ordinal, ev, [d](PJRT_Error_Code* code, std::string* msg) {
+        le->client->post({done, dev->cuda_ordinal, ev, [d](PJRT_Error_Code* code, std::string* msg) {
                             report_expired_wait(d, code, msg);
                           }});
       }
@@ -1334,7 +1304,7 @@ static PJRT_Error* Ext_WaitStream(PJRT_Wait_Until_Buffer_Ready_On_Stream_Args* a
   B2X_RETURN_IF_ERROR(check_live(b));
   await_definition(b);
   B2X_CUDA(cudaSetDevice(b->device->cuda_ordinal));
-  if (b->ready) B2X_CUDA(cudaStreamWaitEvent((cudaStream_t)a->stream, b->ready, 0));
+  B2X_CUDA(wait_mark((cudaStream_t)a->stream, b->ready));
   return nullptr;
 }
 
@@ -1443,8 +1413,7 @@ static void finish_definition(PJRT_Buffer* b, PJRT_Error_Code code, const std::s
   PJRT_Device* dev = b->device;
   cudaSetDevice(dev->cuda_ordinal);
   if (code == PJRT_Error_Code_OK) {
-    cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming);
-    cudaEventRecord(b->ready, dev->h2d);
+    mark_stream(dev->h2d, &b->ready);
   } else {
     b->err_code = code;
     b->err_msg = msg;
@@ -1458,10 +1427,7 @@ static void finish_definition(PJRT_Buffer* b, PJRT_Error_Code code, const std::s
   d->cv.notify_all();
   for (PJRT_Event* ev : waiters) {
     if (code != PJRT_Error_Code_OK) { ev->set(code, msg); ev->unref(); continue; }
-    cudaEvent_t e2;
-    cudaEventCreateWithFlags(&e2, cudaEventDisableTiming);
-    cudaEventRecord(e2, dev->h2d);
-    b->client->post({e2, dev->cuda_ordinal, ev, nullptr});
+    b->client->post({b->ready, dev->cuda_ordinal, ev, nullptr});
     ev->unref();                                              // the waiter list's reference
   }
 }
@@ -1538,10 +1504,9 @@ static PJRT_Error* transfer_into(PJRT_AsyncHostToDeviceTransferManager* tm, int 
   B2X_CUDA(cudaSetDevice(dev->cuda_ordinal));
   if (size) B2X_CUDA(cudaMemcpyAsync((char*)b->ptr + offset, data, (size_t)size, cudaMemcpyHostToDevice, dev->h2d));
   PJRT_Event* ev = new PJRT_Event();
-  cudaEvent_t ce;
-  cudaEventCreateWithFlags(&ce, cudaEventDisableTiming);
-  cudaEventRecord(ce, dev->h2d);
-  tm->client->post({ce, dev->cuda_ordinal, ev, nullptr});
+  MarkRef copied;
+  mark_stream(dev->h2d, &copied);
+  tm->client->post({copied, dev->cuda_ordinal, ev, nullptr});
   *done = ev;
   if (last) { s.finished = true; finish_definition(b, PJRT_Error_Code_OK, ""); }
   return nullptr;

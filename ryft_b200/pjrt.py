@@ -195,9 +195,8 @@ A = {
                                                                                             ("serialized_device_assignment", _vp), ("deleter", _vp)]),
     "LoadedExecutable_Delete": _args("LoadedExecutable_Delete", [("executable", _vp)]),
     "LoadedExecutable_IsDeleted": _args("LoadedExecutable_IsDeleted", [("executable", _vp), ("is_deleted", _b)]),
-    "LoadedExecutable_Execute": _args("LoadedExecutable_Execute", [("executable", _vp), ("options", _vp), ("argument_lists", C.POINTER(C.POINTER(_vp))),
-                                                                    ("num_devices", _sz), ("num_args", _sz), ("output_lists", C.POINTER(C.POINTER(_vp))),
-                                                                    ("device_complete_events", C.POINTER(_vp)), ("execute_device", _vp)]),
+    "LoadedExecutable_Execute": _args("LoadedExecutable_Execute", [("executable", _vp), ("options", _vp), ("argument_lists", _vp), ("num_devices", _sz),
+                                                                    ("num_args", _sz), ("output_lists", _vp), ("device_complete_events", _vp), ("execute_device", _vp)]),
     "Buffer_Destroy": _args("Buffer_Destroy", [("buffer", _vp)]),
     "Buffer_Delete": _args("Buffer_Delete", [("buffer", _vp)]),
     "Buffer_IsDeleted": _args("Buffer_IsDeleted", [("buffer", _vp), ("is_deleted", _b)]),
@@ -286,6 +285,8 @@ class Api:
         for i, n in enumerate(names):
             off = 16 + C.sizeof(ApiVersionC) + 8 * i
             self.fns[n] = C.c_void_p.from_address(base + 8 * i).value if off < self.struct_size else None
+        self._callables: Dict[str, Callable[[int], int]] = {}
+        self._extensions: Dict[int, Optional[int]] = {}
 
     def has(self, name: str) -> bool:
         return bool(self.fns.get("PJRT_" + name))
@@ -293,25 +294,27 @@ class Api:
     def extension(self, type_id: int) -> Optional[int]:
         """Address of the extension struct with the given type id in the PJRT_Api::extension_start chain
         (crates/ryft-pjrt/src/lib.rs:205-212), or None; absence maps to Unimplemented in ryft."""
+        if type_id in self._extensions:      # the chain belongs to the plugin and never changes
+            return self._extensions[type_id]
         node = C.c_void_p.from_address(self.ptr + 8).value
         while node:
-            ext_type = C.c_uint.from_address(node + 8).value
-            if ext_type == type_id:
-                return node
+            if C.c_uint.from_address(node + 8).value == type_id:
+                break
             node = C.c_void_p.from_address(node + 16).value
-        return None
+        self._extensions[type_id] = node
+        return node
 
     def call(self, name: str, args) -> None:
         """Invokes PJRT_<name>(&args); a NULL entry maps to UNIMPLEMENTED like ryft's macros do
         (crates/ryft-pjrt/src/macros.rs:36-44)."""
-        fp = self.fns.get("PJRT_" + name)
-        if not fp:
-            raise PjrtError(12, f"PJRT_{name} is not implemented by this plugin")
+        fn = self._callables.get(name)
+        if fn is None:
+            fp = self.fns.get("PJRT_" + name)
+            if not fp:
+                raise PjrtError(12, f"PJRT_{name} is not implemented by this plugin")
+            fn = self._callables[name] = (_VOIDFN if name in ("Error_Destroy", "Error_Message") else _FN)(fp)
         args.struct_size = C.sizeof(args)
-        if name in ("Error_Destroy", "Error_Message"):
-            _VOIDFN(fp)(C.addressof(args))
-            return
-        err = _FN(fp)(C.addressof(args))
+        err = fn(C.addressof(args))
         if err:
             raise self._take_error(err)
 
@@ -621,9 +624,11 @@ class Buffer:
         ext = self.api.extension(EXTENSION_TYPE_STREAM)
         if not ext:
             raise PjrtError(12, "the plugin has no stream extension")
-        fn = C.c_void_p.from_address(ext + 32).value
+        fn = self.api._callables.get("stream extension: wait")
+        if fn is None:
+            fn = self.api._callables["stream extension: wait"] = _FN(C.c_void_p.from_address(ext + 32).value)
         a = _WaitStreamArgs(); a.struct_size = C.sizeof(a); a.stream = stream; a.buffer = self.handle
-        err = _FN(fn)(C.addressof(a))
+        err = fn(C.addressof(a))
         if err:
             raise self.api._take_error(err)
 
@@ -869,23 +874,26 @@ class LoadedExecutable:
             if len(di.inputs) != num_args:
                 raise PjrtError(3, f"device {i} was given {len(di.inputs)} arguments but device 0 was given {num_args}")
         nd = len(inputs)
-        arg_rows = [(_vp * max(num_args, 1))(*[b.handle for b in di.inputs]) for di in inputs]
-        arg_lists = (C.POINTER(_vp) * nd)(*[C.cast(r, C.POINTER(_vp)) for r in arg_rows])
-        out_rows = [(_vp * max(num_outputs, 1))() for _ in range(nd)]
-        out_lists = (C.POINTER(_vp) * nd)(*[C.cast(r, C.POINTER(_vp)) for r in out_rows])
+        # addresses go into the arrays as plain integers: the arrays themselves live until the call has returned
+        arg_rows = [(_vp * num_args)(*[b.handle for b in di.inputs]) for di in inputs]
+        arg_lists = (_vp * nd)(*[C.addressof(r) for r in arg_rows])
+        out_rows = [(_vp * num_outputs)() for _ in range(nd)]
+        out_lists = (_vp * nd)(*[C.addressof(r) for r in out_rows])
         events = (_vp * nd)()
+        kept = getattr(self, "_kept_inputs", None)
+        if kept is None or len(kept) != num_args:      # no argument is donated; the plugin only reads the list
+            kept = self._kept_inputs = (_i64 * num_args)(*range(num_args))
         opts = ExecuteOptionsC(); opts.struct_size = C.sizeof(opts); opts.launch_id = launch_id
-        nd_idx = (_i64 * max(num_args, 1))(*range(num_args))
-        opts.non_donatable_input_indices = C.cast(nd_idx, C.POINTER(_i64)); opts.num_non_donatable_input_indices = num_args
+        opts.non_donatable_input_indices = kept; opts.num_non_donatable_input_indices = num_args
         a = A["LoadedExecutable_Execute"]()
         a.executable = self.handle; a.options = C.addressof(opts)
-        a.argument_lists = C.cast(arg_lists, C.POINTER(C.POINTER(_vp))); a.num_devices = nd; a.num_args = num_args
-        a.output_lists = C.cast(out_lists, C.POINTER(C.POINTER(_vp))); a.device_complete_events = C.cast(events, C.POINTER(_vp))
+        a.argument_lists = C.addressof(arg_lists); a.num_devices = nd; a.num_args = num_args
+        a.output_lists = C.addressof(out_lists); a.device_complete_events = C.addressof(events)
         a.execute_device = execute_device.handle if execute_device else None
         self.api.call("LoadedExecutable_Execute", a)
         res = []
         for d in range(nd):
-            outs = [Buffer(self.client, out_rows[d][o]) for o in range(num_outputs)]
+            outs = [Buffer(self.client, h) for h in out_rows[d]]
             res.append(ExecutionDeviceOutputs(Event(self.api, events[d]), outs))
         return res
 
