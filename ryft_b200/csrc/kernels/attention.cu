@@ -5,13 +5,12 @@
 // (builders: crates/ryft-mlir/src/dialects/stable_hlo/operations/linear_algebra.rs:756-797, functional.rs:188-219,
 // comparison.rs:136-164, control_flow.rs:263) and replaces it with this kernel; no score tensor touches HBM.
 //
-// Two kernels live here.  k_attention_pw (further down; the default) is persistent: one CTA per SM, two workers per CTA,
-// each walking whole query tiles.  k_attention, described next, is the earlier one-tile-per-CTA form, kept as the
-// fallback and for comparison (B2X_ATTENTION_KERNEL=tile).
+// Two kernels live here.  k_attention_pw (further down) is persistent: one CTA per SM, two workers per CTA, each walking
+// whole query tiles.  k_attention, described next, is the one-tile-per-CTA form.  b2x_launch_attention says which problem
+// takes which.
 //
-// k_attention: one CTA per (batch*head, 128-row query tile); the tiles of one head are adjacent in the grid (K/V reuse in L2),
-// longest causal prefix first.  The key blocks of a tile (128 keys each) are dealt alternately to two independent
-// softmax streams: stream s owns blocks j = s, s + 2, ..., its own score buffer, probability buffer, K/V stage and
+// k_attention: one CTA per (batch*head, 128-row query tile), in the order of attn_tile.  The key blocks of a tile (128 keys
+// each) are dealt alternately to two independent softmax streams: stream s owns blocks j = s, s + 2, ..., its own score buffer, probability buffer, K/V stage and
 // output accumulator, and keeps its own running (max, sum).  While one stream exponentiates, the tensor pipe works
 // for the other; the two partial results are merged once, at the end.  96 + 256 * TPR threads:
 //   warp 0      TMA producer: Q once, then K_j and V_j into stage j & 1 as soon as that stage's previous K (after its
@@ -41,10 +40,24 @@ struct AttnParams {
   int64_t BH, Sq, Sk;
   int32_t n_q_tiles;
   int32_t causal;
+  int32_t group_heads;   // heads whose tiles are dealt out together (attn_tile)
   float scale_log2;   // scale * log2(e)
   __nv_bfloat16* out;
   uint32_t idesc_qk, idesc_pv;
 };
+
+// The query tile behind position t: groups of heads whose K and V stay in L2 together, inside a group the tiles with the
+// longest causal prefix of all its heads first.  Dealing out one head after the other left the launch waiting for the last
+// head's longest tile (causal, 128 wide, persistent form: 16 heads of 4096 119 -> 84 us, 32 heads 194 -> 158, 128 heads
+// 636 -> 593).
+__device__ __forceinline__ void attn_tile(const AttnParams& p, int t, int& bh, int& qt) {
+  const int per_group = p.group_heads * p.n_q_tiles;
+  const int g = t / per_group, in = t - g * per_group;
+  const int heads = min(p.group_heads, (int)p.BH - g * p.group_heads);
+  const int rank = in / heads;
+  bh = g * p.group_heads + (in - rank * heads);
+  qt = p.n_q_tiles - 1 - rank;
+}
 
 constexpr int AT_M = 128;   // query rows per CTA
 constexpr int AT_N = 128;   // keys per block
@@ -121,10 +134,8 @@ k_attention(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   auto merge_slot = [&](int s, int half, int row) -> float2* { return (float2*)(smem + SM::P_OFF + s * SM::P_BYTES) + half * AT_M + row; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // consecutive CTAs are the query tiles of one (batch, head), longest causal prefix first: they run together and find
-  // that head's K and V in L2
-  const int bh = (int)(blockIdx.x / p.n_q_tiles);
-  const int qt = p.n_q_tiles - 1 - (int)(blockIdx.x % p.n_q_tiles);
+  int bh, qt;
+  attn_tile(p, (int)blockIdx.x, bh, qt);
   const int q0 = qt * AT_M;
   int64_t k_end = p.Sk;
   if (p.causal && (int64_t)q0 + AT_M < k_end) k_end = (int64_t)q0 + AT_M;
@@ -276,8 +287,8 @@ k_attention(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
       if (!mbar_wait(bar_sf + 8 * s, (uint32_t)(it & 1), abort_flag, status, 17)) { ok = false; break; }
       tc_fence_after();
       // columns of this block that this row may attend to: [0, lim]
-      int64_t lim = p.Sk - 1 - (int64_t)j * AT_N;
-      if (p.causal) { const int64_t c = qrow - (int64_t)j * AT_N; lim = c < lim ? c : lim; }
+      int lim = (int)min(p.Sk - 1 - (int64_t)j * AT_N, (int64_t)AT_N);
+      if (p.causal) lim = min(lim, q0 + row - j * AT_N);
       const bool need_mask = __any_sync(0xffffffffu, lim < AT_N - 1);
       uint32_t r[KC][32];
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
@@ -534,10 +545,10 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // tile t: consecutive tiles are the query tiles of one (batch, head), longest causal prefix first
   auto decode = [&](int t, int& bh, int& q0, int& nblk) {
-    bh = t / p.n_q_tiles;
-    q0 = (p.n_q_tiles - 1 - t % p.n_q_tiles) * AT_M;
+    int qt;
+    attn_tile(p, t, bh, qt);
+    q0 = qt * AT_M;
     int64_t k_end = p.Sk;
     if (p.causal && (int64_t)q0 + AT_M < k_end) k_end = (int64_t)q0 + AT_M;
     nblk = (int)((k_end + AT_N - 1) / AT_N);
@@ -703,8 +714,8 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
         if (!mbar_wait(bar_sf, sc & 1, abort_flag, status, 17)) { ok = false; break; }
         tc_fence_after();
         // columns of this block that this row may attend to: [0, lim]
-        int64_t lim = p.Sk - 1 - (int64_t)it * AT_N;
-        if (p.causal) { const int64_t c = qrow - (int64_t)it * AT_N; lim = c < lim ? c : lim; }
+        int lim = (int)min(p.Sk - 1 - (int64_t)it * AT_N, (int64_t)AT_N);
+        if (p.causal) lim = min(lim, q0 + row - it * AT_N);
         const bool need_mask = __any_sync(0xffffffffu, lim < AT_N - 1);
         uint32_t r[4][32];
 #pragma unroll
@@ -818,6 +829,12 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
 int32_t* sched_slot(cudaStream_t stream);   // defined in gemm_tc.cu: a (tile counter, finished CTAs) pair per stream
 
+// K and V of a group of heads ~ 32 MiB, a quarter of the 126 MB L2.
+static int attn_group_heads(const B2xAttentionArgs* a) {
+  const int64_t n = (32ll << 20) / (a->Sk * a->D * 4);
+  return (int)(n < 1 ? 1 : (n > a->BH ? a->BH : n));
+}
+
 // Returns -1 when the stream has no scheduler pair (the caller then uses the one-tile-per-CTA form).
 template <int D>
 static int launch_attention_pw(const B2xAttentionArgs* a, int32_t* status, cudaStream_t stream) {
@@ -832,6 +849,7 @@ static int launch_attention_pw(const B2xAttentionArgs* a, int32_t* status, cudaS
   AttnParams p{};
   p.BH = a->BH; p.Sq = a->Sq; p.Sk = a->Sk;
   p.n_q_tiles = (int)((a->Sq + AT_M - 1) / AT_M);
+  p.group_heads = attn_group_heads(a);
   p.causal = a->causal;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   p.out = (__nv_bfloat16*)a->o;
@@ -868,6 +886,7 @@ static int launch_attention(const B2xAttentionArgs* a, int32_t* status, cudaStre
   AttnParams p{};
   p.BH = a->BH; p.Sq = a->Sq; p.Sk = a->Sk;
   p.n_q_tiles = (int)((a->Sq + AT_M - 1) / AT_M);
+  p.group_heads = attn_group_heads(a);
   p.causal = a->causal;
   p.scale_log2 = a->scale * 1.4426950408889634f;
   p.out = (__nv_bfloat16*)a->o;
@@ -899,16 +918,25 @@ extern "C" int b2x_launch_attention(const B2xAttentionArgs* a, int32_t* status, 
   cudaStream_t stream = (cudaStream_t)stream_;
   if (a->BH <= 0 || a->Sq <= 0 || a->Sk <= 0) return (int)cudaErrorInvalidValue;
   if (((uintptr_t)a->q & 15) || ((uintptr_t)a->k & 15) || ((uintptr_t)a->v & 15) || ((uintptr_t)a->o & 15)) return (int)cudaErrorInvalidValue;
-  // Variants kept for comparison, both measured slower on the 4096 x 128 causal case (0.85 ms and 0.72 ms against 0.68 ms):
-  // B2X_ATTENTION_P=tmem (probabilities through TMEM as the second MMA's A operand: frees the P buffers, but a stream's next
-  // score block must then wait for its P V product), B2X_ATTENTION_THREADS_PER_ROW=2 (two threads share a query row)
-  // The persistent two-worker form is the default (0.64 ms on the 4096 x 128 causal case against 0.68 ms);
-  // B2X_ATTENTION_KERNEL=tile selects the one-tile-per-CTA form and its variants below.
+  // Which form: the persistent two-worker kernel hides a tile's start-up and write-out behind the other worker, the
+  // one-tile-per-CTA kernel puts both halves of the SM on one tile and runs a little faster per key block.  So the latter
+  // takes problems that would leave a worker at most one tile (two per SM), where it halves the longest tile's time, and
+  // unmasked ones of 128-wide heads with tiles of 16 and more key blocks.  Device times, persistent / one-tile:
+  //   causal, 128 wide: 29 heads x 512 20.9 / 12.3 us, 8 x 4096 84 / 45, 16 x 4096 84 / 86, 32 x 4096 158 / 172, 128 x 4096 592 / 661
+  //   unmasked: 32 x 4096 x 128 313 / 283, 64 x 2048 x 128 171 / 164, 32 x 2048 x 64 76 / 82, 24 x 1000 x 64 26.5 / 26.7
+  // B2X_ATTENTION_KERNEL=tile / persistent selects one of them.
   const char* form = getenv("B2X_ATTENTION_KERNEL");
-  if (!(form && form[0] == 't') && (a->D == 128 || a->D == 64)) {
+  const int64_t tiles = (a->Sq + AT_M - 1) / AT_M * a->BH;
+  bool one_tile = tiles <= 2 * kNumSms || (!a->causal && a->D == 128 && a->Sk > 15 * AT_N);
+  if (form && (form[0] == 't' || form[0] == 'p')) one_tile = form[0] == 't';
+  if (!one_tile && (a->D == 128 || a->D == 64)) {
     const int rc = a->D == 128 ? launch_attention_pw<128>(a, status, stream) : launch_attention_pw<64>(a, status, stream);
     if (rc != -1) return rc;
   }
+  // Variants of the one-tile form kept for comparison, both measured slower on the 4096 x 128 causal case (0.85 ms and 0.72 ms
+  // against 0.68 ms): B2X_ATTENTION_P=tmem (probabilities through TMEM as the second MMA's A operand: frees the P buffers, but
+  // a stream's next score block must then wait for its P V product), B2X_ATTENTION_THREADS_PER_ROW=2 (two threads share a
+  // query row).
   const char* tpr = getenv("B2X_ATTENTION_THREADS_PER_ROW");
   const char* pv = getenv("B2X_ATTENTION_P");
   const bool two = tpr && tpr[0] == '2';
