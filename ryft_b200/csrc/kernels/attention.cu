@@ -160,7 +160,7 @@ k_attention(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
 
   if (warp == 0) {
     // ---------------------------------------------- TMA producer --------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(bar_q, SM::Q_BYTES);
 #pragma unroll
       for (int c = 0; c < DC; c++) tma_load_3d(sbase + SM::Q_OFF + c * CHUNK_BYTES, &tmQ, bar_q, c * 64, q0, bh);
@@ -205,7 +205,7 @@ k_attention(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     // ---------------------------------------------- MMA issuers -----------------------------------------------------
     // One issuing thread per stream, so that a stream whose probabilities are late never holds up the other stream's
     // next score block.  The two threads touch disjoint TMEM columns and shared-memory buffers (Q is only read).
-    if (lane == 0) {
+    if (elect_one()) {
       const int s = warp - 1;
       const int n_mine = nblk > s ? (nblk - s + 1) / 2 : 0;
       bool ok = mbar_wait(bar_q, 0, abort_flag, status, 12);
@@ -556,7 +556,7 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
 
   if (warp < 2) {
     // ---------------------------------------------- TMA producer --------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t kc = 0, vc = 0;       // K and V blocks loaded so far
       bool ok = true;
       for (int n = 0; ok; n++) {
@@ -602,7 +602,7 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
     }
   } else if (warp < 4) {
     // ---------------------------------------------- MMA issuer ------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t kc = 0, vc = 0, hc = 0;     // score blocks issued, V blocks consumed, P V half-steps issued
       const uint32_t s_tmem = tmem_base + (uint32_t)(w * 128), o_tmem = tmem_base + 256u + (uint32_t)(w * D);
       const uint32_t qa = wbase + SM::Q_OFF, ka = wbase + SM::K_OFF, va = wbase + SM::V_OFF, pa = wbase + SM::P_OFF;

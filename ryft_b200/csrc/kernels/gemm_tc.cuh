@@ -194,7 +194,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer ------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -256,7 +256,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer ----------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -395,7 +395,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 // one before that
                 const uint32_t stg = stg_sel ? stg1 : stg0;
                 const uint32_t my = stg + (uint32_t)lane * 64u;
-                if (lane == 0) { if (p.short_k) bulk_wait_read_1(); else bulk_wait_read(); }
+                if (elect_one()) { if (p.short_k) bulk_wait_read_1(); else bulk_wait_read(); }
                 __syncwarp();
 #pragma unroll
                 for (int v = strip * (STRIP / 8); v < (strip + 1) * (STRIP / 8); v++) {
@@ -412,7 +412,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                 fence_async_shared();
                 __syncwarp();
                 const bool do_store = n0 + c * 32 + strip * STRIP < p.N && m0 + quad * 32 < p.M;   // the same for the whole warp
-                if (lane == 0 && do_store) {
+                if (do_store && elect_one()) {
                   tma_store_3d(&tmOut, stg, n0 + c * 32 + strip * STRIP, m0 + quad * 32, b);
                   bulk_commit();
                 }
@@ -476,7 +476,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
   }
 
   if constexpr (tc_tma_store_epilogue<ID>()) {
-    if (warp >= 2 && lane == 0) bulk_wait_all();   // this thread's result stores are complete before the CTA retires
+    __syncwarp();
+    if (warp >= 2 && elect_one()) bulk_wait_all();   // this thread's result stores are complete before the CTA retires
   }
   tc_fence_before();
   __syncthreads();
