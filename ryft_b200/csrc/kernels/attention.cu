@@ -157,6 +157,8 @@ k_attention(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();          // everything above touched this SM only
 
   if (warp == 0) {
     // ---------------------------------------------- TMA producer --------------------------------------------------
@@ -544,6 +546,8 @@ k_attention_pw(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();          // everything above touched this SM only
 
   auto decode = [&](int t, int& bh, int& q0, int& nblk) {
     int qt;
@@ -870,7 +874,8 @@ static int launch_attention_pw(const B2xAttentionArgs* a, int32_t* status, cudaS
   if (tiles <= 0) return 0;
   if (tiles > 0x7fffff00) return (int)cudaErrorInvalidValue;
   const int64_t ctas = (tiles + 1) / 2 < kNumSms ? (tiles + 1) / 2 : kNumSms;
-  kern<<<(unsigned)ctas, 384, SM::TOTAL, stream>>>(tmQ, tmK, tmV, p, sched, status);
+  const cudaError_t e = launch_overlapped(kern, dim3((unsigned)ctas), dim3(384), SM::TOTAL, stream, tmQ, tmK, tmV, p, sched, status);
+  if (e != cudaSuccess) return (int)e;
   count_launch();
   return (int)cudaGetLastError();
 }
@@ -906,7 +911,8 @@ static int launch_attention(const B2xAttentionArgs* a, int32_t* status, cudaStre
   const int64_t grid = (int64_t)p.n_q_tiles * a->BH;
   if (grid <= 0) return 0;
   if (grid > 0x7fffffff) return (int)cudaErrorInvalidValue;
-  kern<<<(unsigned)grid, 96 + 256 * TPR, SM::TOTAL, stream>>>(tmQ, tmK, tmV, p, status);
+  const cudaError_t e = launch_overlapped(kern, dim3((unsigned)grid), dim3(96 + 256 * TPR), SM::TOTAL, stream, tmQ, tmK, tmV, p, status);
+  if (e != cudaSuccess) return (int)e;
   count_launch();
   return (int)cudaGetLastError();
 }

@@ -13,6 +13,8 @@ std::atomic<int64_t> g_launch_count{0};
 
 template <int V, int ID>
 __global__ void __launch_bounds__(256) k_elementwise(const __grid_constant__ B2xVmProgram P, uint64_t n_vec) {
+  pdl_trigger();
+  pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   uint32_t zero[V];
 #pragma unroll
@@ -36,16 +38,18 @@ extern "C" int b2x_launch_elementwise(const B2xVmProgram* prog, int64_t n_elemen
   uint64_t cap = (uint64_t)kNumSms * 8 * 4;
   if (blocks > cap) blocks = cap;
   dim3 grid((unsigned)blocks), block(256);
+  cudaError_t e;
   if (vec == 8) {
     // a program whose structure was known at build time runs as straight-line code, anything else is interpreted
     switch (vm_static_enabled() ? vm_static_lookup(vm_signature_hash(*prog)) : 0) {
-#define X(I) case I: k_elementwise<8, I><<<grid, block, 0, stream>>>(*prog, n_vec); break;
+#define X(I) case I: e = launch_overlapped(k_elementwise<8, I>, grid, block, 0, stream, *prog, n_vec); break;
       B2X_VM_STATIC_ELEMENTWISE(X)
 #undef X
-      default: k_elementwise<8, 0><<<grid, block, 0, stream>>>(*prog, n_vec); break;
+      default: e = launch_overlapped(k_elementwise<8, 0>, grid, block, 0, stream, *prog, n_vec); break;
     }
-  } else if (vec == 4) k_elementwise<4, 0><<<grid, block, 0, stream>>>(*prog, n_vec);
-  else k_elementwise<1, 0><<<grid, block, 0, stream>>>(*prog, n_vec);
+  } else if (vec == 4) e = launch_overlapped(k_elementwise<4, 0>, grid, block, 0, stream, *prog, n_vec);
+  else e = launch_overlapped(k_elementwise<1, 0>, grid, block, 0, stream, *prog, n_vec);
+  if (e != cudaSuccess) return (int)e;
   count_launch();
   return (int)cudaGetLastError();
 }

@@ -53,6 +53,8 @@ __device__ __forceinline__ void split_write(float* o, int64_t K, int64_t k, floa
 }
 __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B) {
   __shared__ float tile[32][33];
+  pdl_trigger();
+  pdl_wait();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t total = A.n_tiles + B.n_tiles;
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -108,7 +110,8 @@ extern "C" int b2x_launch_split_f32(const B2xGemmArgs* a, float* a_split, float*
   int64_t grid = A.n_tiles + B.n_tiles;
   if (grid > (int64_t)kNumSms * 8) grid = (int64_t)kNumSms * 8;
   if (grid < 1) return 0;
-  k_split_f32<<<(unsigned)grid, 256, 0, stream>>>(A, B);
+  const cudaError_t e = launch_overlapped(k_split_f32, dim3((unsigned)grid), dim3(256), 0, stream, A, B);
+  if (e != cudaSuccess) return (int)e;
   count_launch(1);
   return (int)cudaGetLastError();
 }

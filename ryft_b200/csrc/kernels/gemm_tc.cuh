@@ -186,6 +186,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();          // everything above touched this SM only
   // stage geometry: the ring is STAGES * STAGE_BYTES either way (tall tiles are only routed to the <256, 4> kernels,
   // whose 4 x 48 KB ring is 3 x 64 KB)
   const int n_stages = (p.tall || p.short_k) ? 3 : STAGES;
@@ -554,7 +556,8 @@ static int launch_tc(const CUtensorMap& tmA, const CUtensorMap& tmB, const TcPar
   // Tile = CTA where the CTAs leave 32 SMs free: one that has to wait for its SM (a collective's CTAs may hold up to that
   // many) would hold up the launch, where the counter lets the others take its share.
   p.one_tile = p.num_tiles <= kNumSms - 32 ? 1 : 0;
-  kern<<<(unsigned)grid, TC_THREADS, SM::TOTAL, stream>>>(tmA, tmB, tmOut, p, epi, status);
+  const cudaError_t e = launch_overlapped(kern, dim3((unsigned)grid), dim3(TC_THREADS), SM::TOTAL, stream, tmA, tmB, tmOut, p, epi, status);
+  if (e != cudaSuccess) return (int)e;
   count_launch();
   return (int)cudaGetLastError();
 }

@@ -221,6 +221,8 @@ __global__ void __launch_bounds__(256, ID != 0 ? 4 : 1) k_reduce_rows(const __gr
   __shared__ uint32_t smem[8];
   __shared__ int s_last;
   constexpr int PIECES_PER_CTA = 256 / T;
+  pdl_trigger();
+  pdl_wait();
   const int lane_in_piece = threadIdx.x % T;
   const int64_t n_pieces = K.A * K.S;
   uint32_t zero[V];
@@ -329,6 +331,8 @@ __global__ void __launch_bounds__(256) k_reduce_rows_direct(const char* __restri
                                                             const __grid_constant__ B2xVmProgram Q) {
   __shared__ uint32_t smem[8];
   __shared__ int s_last;
+  pdl_trigger();
+  pdl_wait();
   const int64_t n_pieces = K.A * K.S;
   const uint32_t ident = red_identity(K.monoid, K.cls);
   auto fold8 = [&](float& t, const uint4& lo, const uint4& hi) {
@@ -420,6 +424,8 @@ __global__ void __launch_bounds__(256) k_reduce_cols(const __grid_constant__ B2x
                                                      const char* __restrict__ base, int n_bblocks, int CL) {
   namespace cg = cooperative_groups;
   __shared__ uint32_t smem[256 * V];
+  pdl_trigger();
+  pdl_wait();
   const int BX = blockDim.x, RY = blockDim.y;
   const int rank = CL > 1 ? (int)(blockIdx.x % (unsigned)CL) : 0;
   const int64_t n_work = K.A * K.S * (int64_t)n_bblocks;
@@ -542,11 +548,13 @@ static int launch_cols(const B2xVmProgram& P, const ReduceKArgs& K, const B2xVmP
   cfg.gridDim = dim3((unsigned)(clusters * CL));
   cfg.blockDim = dim3((unsigned)bx, (unsigned)ry);
   cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)CL; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
+  cudaLaunchAttribute attr[2]{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)CL; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
   const char* base = (const char*)P.tensors[0].ptr;
   return (int)cudaLaunchKernelEx(&cfg, k_reduce_cols<V, DIRECT, MC>, P, K, Q, base, n_bblocks, CL);
 }
@@ -568,23 +576,26 @@ static int launch_one(const B2xVmProgram& P, ReduceKArgs K, const B2xVmProgram& 
       if (dk) {
         const char* base = (const char*)P.tensors[0].ptr;
         const bool f32 = P.tensors[0].elem == EL_F32;
-#define B2X_DIRECT(ES_, SQ_, MC_) k_reduce_rows_direct<ES_, SQ_, MC_><<<grid, block, 0, stream>>>(base, K, Q)
+        cudaError_t e;
+#define B2X_DIRECT(ES_, SQ_, MC_) e = launch_overlapped(k_reduce_rows_direct<ES_, SQ_, MC_>, grid, block, 0, stream, base, K, Q)
         if (f32) { if (dk == 2) { if (mc0 == 1) B2X_DIRECT(4, true, 1); else B2X_DIRECT(4, true, 2); } else { if (mc0 == 1) B2X_DIRECT(4, false, 1); else B2X_DIRECT(4, false, 2); } }
         else { if (dk == 2) { if (mc0 == 1) B2X_DIRECT(2, true, 1); else B2X_DIRECT(2, true, 2); } else { if (mc0 == 1) B2X_DIRECT(2, false, 1); else B2X_DIRECT(2, false, 2); } }
 #undef B2X_DIRECT
+        if (e != cudaSuccess) return (int)e;
         count_launch();
         return (int)cudaGetLastError();
       }
     }
 #define B2X_ROWS_MC(VV, II, MM)                                                           \
-    if (warp_rows) k_reduce_rows<VV, 32, II, MM><<<grid, block, 0, stream>>>(P, K, Q);    \
-    else k_reduce_rows<VV, 256, II, MM><<<grid, block, 0, stream>>>(P, K, Q);
+    if (warp_rows) err = launch_overlapped(k_reduce_rows<VV, 32, II, MM>, grid, block, 0, stream, P, K, Q);    \
+    else err = launch_overlapped(k_reduce_rows<VV, 256, II, MM>, grid, block, 0, stream, P, K, Q);
     // specialised programs also get a combine fixed at compile time for f32 sum / f32 max
 #define B2X_ROWS(VV, II)                                                                  \
     if (II != 0 && mc == 1) { B2X_ROWS_MC(VV, II, (II != 0 ? 1 : 0)) }                    \
     else if (II != 0 && mc == 2) { B2X_ROWS_MC(VV, II, (II != 0 ? 2 : 0)) }               \
     else { B2X_ROWS_MC(VV, II, 0) }
     const int mc = red_combine_class(K.monoid, K.cls);
+    cudaError_t err;
     if (vec == 8) {
       switch (vm_static_enabled() ? vm_static_lookup(vm_signature_hash(P)) : 0) {
 #define X(I) case I: B2X_ROWS(8, I) break;
@@ -595,6 +606,7 @@ static int launch_one(const B2xVmProgram& P, ReduceKArgs K, const B2xVmProgram& 
     } else if (vec == 4) { B2X_ROWS(4, 0) } else { B2X_ROWS(1, 0) }
 #undef B2X_ROWS_MC
 #undef B2X_ROWS
+    if (err != cudaSuccess) return (int)err;
   } else {
     const int mc = red_combine_class(K.monoid, K.cls);
     const int es = (mc == 1 || mc == 2) && vm_static_enabled() ? direct_cols(P, K) : 0;

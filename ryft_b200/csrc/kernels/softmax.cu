@@ -31,6 +31,8 @@ __global__ void __launch_bounds__(T == 32 ? 256 : T) k_softmax_rows(const float*
   __shared__ float smem[2][T / 32];
   constexpr int ROWS = T == 32 ? 8 : 1;
   constexpr int P = E / V;                              // pieces per thread
+  pdl_trigger();
+  pdl_wait();
   const int tid = T == 32 ? (threadIdx.x & 31) : threadIdx.x;
   // a row's threads leave together: with T == 32 they are one warp, otherwise the whole CTA
   for (int64_t row = (int64_t)blockIdx.x * ROWS + (T == 32 ? threadIdx.x >> 5 : 0); row < rows; row += (int64_t)gridDim.x * ROWS) {
@@ -103,10 +105,12 @@ static int launch_rows(const float* x, char* out, uint8_t elem, int64_t rows, in
   int64_t grid = (rows + ROWS - 1) / ROWS;
   if (grid > (int64_t)kNumSms * 512) grid = (int64_t)kNumSms * 512;
   const unsigned block = T == 32 ? 256 : T;
-  if (elem == EL_F32) k_softmax_rows<T, E, V, EL_F32><<<(unsigned)grid, block, 0, stream>>>(x, out, rows, n);
-  else if (elem == EL_BF16) k_softmax_rows<T, E, V, EL_BF16><<<(unsigned)grid, block, 0, stream>>>(x, out, rows, n);
-  else if (elem == EL_F16) k_softmax_rows<T, E, V, EL_F16><<<(unsigned)grid, block, 0, stream>>>(x, out, rows, n);
+  cudaError_t e;
+  if (elem == EL_F32) e = launch_overlapped(k_softmax_rows<T, E, V, EL_F32>, dim3((unsigned)grid), dim3(block), 0, stream, x, out, rows, n);
+  else if (elem == EL_BF16) e = launch_overlapped(k_softmax_rows<T, E, V, EL_BF16>, dim3((unsigned)grid), dim3(block), 0, stream, x, out, rows, n);
+  else if (elem == EL_F16) e = launch_overlapped(k_softmax_rows<T, E, V, EL_F16>, dim3((unsigned)grid), dim3(block), 0, stream, x, out, rows, n);
   else return (int)cudaErrorInvalidValue;
+  if (e != cudaSuccess) return (int)e;
   count_launch();
   return (int)cudaGetLastError();
 }
