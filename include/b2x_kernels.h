@@ -97,6 +97,12 @@ B2X_API int b2x_gemm_tc_route(const B2xGemmArgs* host_args, const B2xVmProgram* 
  * (K-major rows of 3K elements), so that one TF32 GEMM over K' = 3K yields hi*hi + hi*lo + lo*hi. */
 B2X_API int b2x_launch_split_f32(const B2xGemmArgs* host_args, float* a_split, float* b_split, b2x_stream_t stream);
 
+/* f32 dot_general as three TF32 products on the tensor cores: splits both operands (any strides) into scratch, rows of
+ * [hi | lo], and multiplies hi*hi + hi*lo + lo*hi from there.  M, N and the epilogue as for b2x_launch_gemm_tc; `scratch`
+ * holds b2x_gemm_f32_scratch_bytes(batch, M, N, K) bytes and is 16-byte aligned.  Two kernels. */
+B2X_API int64_t b2x_gemm_f32_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K);
+B2X_API int b2x_launch_gemm_f32(const B2xGemmArgs* host_args, const B2xVmProgram* host_epilogue, void* scratch, int32_t* status, b2x_stream_t stream);
+
 /* Fused causal scaled-dot-product attention forward over [BH, S, D] bf16 (the dot_general -> scale -> iota/compare/
  * select mask -> reduce max -> exponential -> reduce add -> divide -> dot_general chain written with the builders
  * cited above). */

@@ -34,13 +34,16 @@ int32_t* sched_slot(cudaStream_t stream) {
 }
 
 // ---- f32 -> hi/lo TF32 split for the 3xTF32 scheme ------------------------------------------------------------------
-// out rows are K-major with 3K elements: sel 0 -> [hi | hi | lo], sel 1 -> [hi | lo | hi].  One launch splits both
+// out rows are K-major: sel 0 -> [hi | hi | lo] and sel 1 -> [hi | lo | hi] with 3K elements, sel 2 -> [hi | lo] with 2 ld
+// elements, each half padded with zeros from K to ld.  One launch splits both
 // operands: a CTA takes 32 x 32 (row, k) tiles of either.  A source that is contiguous along k is read and written
 // with lane = k; any other source is read with lane = row and turned through shared memory, so that the writes are
 // contiguous along k as well.
+// Elements of one half of a paired row: whole k-blocks, so that none straddles the two halves.
+static int64_t paired_ld(int64_t K) { return (K + 31) / 32 * 32; }
 struct SplitSide {
   const float* src; float* dst;
-  int64_t rows, K, sb, sr, sk;
+  int64_t rows, K, ld, pitch, sb, sr, sk;   // ld: elements of a half, pitch: of an output row
   int64_t tiles_r, tiles_k, n_tiles;
   int sel;
 };
@@ -48,6 +51,7 @@ __device__ __forceinline__ void split_write(float* o, int64_t K, int64_t k, floa
   const float hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
   const float lo = __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u);
   o[k] = hi;
+  if (sel == 2) { o[K + k] = lo; return; }
   o[K + k] = sel == 0 ? hi : lo;
   o[2 * K + k] = sel == 0 ? lo : hi;
 }
@@ -66,13 +70,13 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
     const int64_t b = u / S.tiles_r;
     const int64_t r0 = tr * 32, k0 = tk * 32;
     const float* src = S.src + b * S.sb;
-    float* dst = S.dst + b * S.rows * (3 * S.K);
+    float* dst = S.dst + b * S.rows * S.pitch;
     if (S.sk == 1) {
       const int64_t k = k0 + tx;
 #pragma unroll
       for (int i = ty; i < 32; i += 8) {
         const int64_t r = r0 + i;
-        if (r < S.rows && k < S.K) split_write(dst + r * (3 * S.K), S.K, k, __ldg(src + r * S.sr + k), S.sel);
+        if (r < S.rows && k < S.ld) split_write(dst + r * S.pitch, S.ld, k, k < S.K ? __ldg(src + r * S.sr + k) : 0.0f, S.sel);
       }
     } else {
       const int64_t r_in = r0 + tx;
@@ -86,7 +90,7 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
 #pragma unroll
       for (int i = ty; i < 32; i += 8) {
         const int64_t r = r0 + i;
-        if (r < S.rows && k < S.K) split_write(dst + r * (3 * S.K), S.K, k, tile[tx][i], S.sel);
+        if (r < S.rows && k < S.ld) split_write(dst + r * S.pitch, S.ld, k, tile[tx][i], S.sel);
       }
       __syncthreads();
     }
@@ -95,18 +99,18 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
 
 }  // namespace b2x
 
-extern "C" int b2x_launch_split_f32(const B2xGemmArgs* a, float* a_split, float* b_split, b2x_stream_t stream_) {
-  using namespace b2x;
-  cudaStream_t stream = (cudaStream_t)stream_;
+namespace b2x {
+static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bool paired, cudaStream_t stream) {
   if (a->elem != EL_F32) return (int)cudaErrorInvalidValue;
   auto side = [&](const void* src, float* dst, int64_t rows, int64_t sb, int64_t sr, int64_t sk, int sel) {
     SplitSide s{};
     s.src = (const float*)src; s.dst = dst; s.rows = rows; s.K = a->K; s.sb = sb; s.sr = sr; s.sk = sk; s.sel = sel;
+    s.ld = paired ? paired_ld(a->K) : a->K; s.pitch = paired ? 2 * s.ld : 3 * a->K;
     s.tiles_r = (rows + 31) / 32; s.tiles_k = (a->K + 31) / 32; s.n_tiles = a->batch * s.tiles_r * s.tiles_k;
     return s;
   };
-  const SplitSide A = side(a->a, a_split, a->M, a->a_batch_stride, a->a_row_stride, a->a_k_stride, 0);
-  const SplitSide B = side(a->b, b_split, a->N, a->b_batch_stride, a->b_row_stride, a->b_k_stride, 1);
+  const SplitSide A = side(a->a, a_split, a->M, a->a_batch_stride, a->a_row_stride, a->a_k_stride, paired ? 2 : 0);
+  const SplitSide B = side(a->b, b_split, a->N, a->b_batch_stride, a->b_row_stride, a->b_k_stride, paired ? 2 : 1);
   int64_t grid = A.n_tiles + B.n_tiles;
   if (grid > (int64_t)kNumSms * 8) grid = (int64_t)kNumSms * 8;
   if (grid < 1) return 0;
@@ -114,6 +118,11 @@ extern "C" int b2x_launch_split_f32(const B2xGemmArgs* a, float* a_split, float*
   if (e != cudaSuccess) return (int)e;
   count_launch(1);
   return (int)cudaGetLastError();
+}
+}  // namespace b2x
+
+extern "C" int b2x_launch_split_f32(const B2xGemmArgs* a, float* a_split, float* b_split, b2x_stream_t stream) {
+  return b2x::launch_split(a, a_split, b_split, false, (cudaStream_t)stream);
 }
 
 namespace b2x {
@@ -126,7 +135,8 @@ struct TcRoute {
   TcParams p{};
 };
 
-static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, TcRoute* r) {
+// paired: the operands are rows of [hi | lo] (TcParams::paired), K counts one half
+static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bool paired, TcRoute* r) {
   if (a->batch <= 0 || a->M <= 0 || a->N <= 0 || a->K <= 0) return (int)cudaErrorInvalidValue;
   r->tf32 = a->elem == EL_F32;
   if (!r->tf32 && a->elem != EL_BF16 && a->elem != EL_F16) return (int)cudaErrorInvalidValue;
@@ -159,7 +169,9 @@ static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, TcRoute*
   if (p.num_tiles >= (1ll << 31)) return (int)cudaErrorInvalidValue;
   p.k_blocks = (int)((a->K + BK - 1) / BK);
   p.transposed = a->K <= 8192 ? 1 : 0;
-  p.epi_groups = p.k_blocks <= 8 ? 1 : 2;
+  p.paired = paired ? 1 : 0;
+  p.lo_off = paired ? (int32_t)paired_ld(a->K) : 0;
+  p.epi_groups = p.k_blocks * (paired ? 3 : 1) <= 8 ? 1 : 2;
   // Tall (256 x 256) tiles: long-K 16-bit problems whose tall tiles still fill the last round of the 148 SMs.  Their
   // epilogue is not overlapped, so K must be long enough to make it small; B2X_GEMM_TALL=0 / 1 switches them off / forces
   // them wherever the kernel can run them.
@@ -186,7 +198,7 @@ static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, TcRoute*
   }
   {
     // A slab of a group ~ 32 MiB (a quarter of the 126 MB L2)
-    const int64_t slab_per_m_tile = bm * a->K * es;
+    const int64_t slab_per_m_tile = bm * a->K * es * (paired ? 2 : 1);
     int64_t gm = (32ll << 20) / (slab_per_m_tile > 0 ? slab_per_m_tile : 1);
     if (gm < 4) gm = 4;
     if (gm > 64) gm = 64;
@@ -203,7 +215,7 @@ static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, TcRoute*
 extern "C" int b2x_gemm_tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t out[12]) {
   using namespace b2x;
   TcRoute r;
-  int rc = tc_route(a, epilogue, &r);
+  int rc = tc_route(a, epilogue, false, &r);
   if (rc) return rc;
   out[0] = r.BN; out[1] = r.static_id; out[2] = r.p.epi_groups;
   out[3] = (r.static_id && r.p.transposed && tc_static_stores(r.static_id) >= 2) ? 1 : 0;
@@ -215,11 +227,10 @@ extern "C" int b2x_gemm_tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilo
   return 0;
 }
 
-extern "C" int b2x_launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t* status, b2x_stream_t stream_) {
-  using namespace b2x;
-  cudaStream_t stream = (cudaStream_t)stream_;
+namespace b2x {
+static int launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bool paired, int32_t* status, cudaStream_t stream) {
   TcRoute r;
-  int rc = tc_route(a, epilogue, &r);
+  int rc = tc_route(a, epilogue, paired, &r);
   if (rc) return rc;
   if (((uintptr_t)a->a & 15) || ((uintptr_t)a->b & 15)) return (int)cudaErrorInvalidValue;
   const bool tf32 = r.tf32, a_mn = r.a_mn, b_mn = r.b_mn;
@@ -232,15 +243,16 @@ extern "C" int b2x_launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epil
   // B2X_GEMM_LOADS=3d keeps one load per 128-byte-wide sub-tile of an MN-major operand (for comparison)
   static const bool folded = [] { const char* e = getenv("B2X_GEMM_LOADS"); return !(e && e[0] == '3'); }();
   p.a_mn_4d = p.b_mn_4d = 0;
+  const uint64_t k_extent = paired ? 2 * (uint64_t)paired_ld(a->K) : (uint64_t)a->K;
   const uint32_t bm = p.tall ? 2 * TC_BM : TC_BM;   // rows of A per stage
-  if (!a_mn) ok = encode_3d(&tmA, dt, es, a->a, (uint64_t)a->K, (uint64_t)a->M, (uint64_t)a->batch, (uint64_t)a_ld, (uint64_t)a->a_batch_stride, BK, bm);
+  if (!a_mn) ok = encode_3d(&tmA, dt, es, a->a, k_extent, (uint64_t)a->M, (uint64_t)a->batch, (uint64_t)a_ld, (uint64_t)a->a_batch_stride, BK, bm);
   else {
     ok = folded && encode_mn_major_4d(&tmA, dt, es, a->a, (uint64_t)a->M, (uint64_t)a->K, (uint64_t)a->batch, (uint64_t)a_ld, (uint64_t)a->a_batch_stride, CHUNK, BK, bm);
     if (ok) p.a_mn_4d = 1;
     else ok = encode_3d(&tmA, dt, es, a->a, (uint64_t)a->M, (uint64_t)a->K, (uint64_t)a->batch, (uint64_t)a_ld, (uint64_t)a->a_batch_stride, CHUNK, BK);
   }
   if (!ok) return (int)cudaErrorInvalidValue;
-  if (!b_mn) ok = encode_3d(&tmB, dt, es, a->b, (uint64_t)a->K, (uint64_t)a->N, (uint64_t)a->batch, (uint64_t)b_ld, (uint64_t)a->b_batch_stride, BK, BN);
+  if (!b_mn) ok = encode_3d(&tmB, dt, es, a->b, k_extent, (uint64_t)a->N, (uint64_t)a->batch, (uint64_t)b_ld, (uint64_t)a->b_batch_stride, BK, BN);
   else {
     ok = folded && encode_mn_major_4d(&tmB, dt, es, a->b, (uint64_t)a->N, (uint64_t)a->K, (uint64_t)a->batch, (uint64_t)b_ld, (uint64_t)a->b_batch_stride, CHUNK, BK, BN);
     if (ok) p.b_mn_4d = 1;
@@ -263,4 +275,30 @@ extern "C" int b2x_launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epil
   if (BN == 256) return launch_tc<256, 4, false, 0>(tmA, tmB, p, *epilogue, status, stream);
   if (BN == 128) return launch_tc<128, 6, false, 0>(tmA, tmB, p, *epilogue, status, stream);
   return launch_tc<64, 8, false, 0>(tmA, tmB, p, *epilogue, status, stream);
+}
+}  // namespace b2x
+
+extern "C" int b2x_launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t* status, b2x_stream_t stream) {
+  return b2x::launch_gemm_tc(a, epilogue, false, status, (cudaStream_t)stream);
+}
+
+extern "C" int64_t b2x_gemm_f32_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  const int64_t pitch = 2 * b2x::paired_ld(K) * 4;
+  return (batch * M * pitch + 1023) / 1024 * 1024 + batch * N * pitch;
+}
+
+extern "C" int b2x_launch_gemm_f32(const B2xGemmArgs* a, const B2xVmProgram* epilogue, void* scratch, int32_t* status, b2x_stream_t stream_) {
+  using namespace b2x;
+  cudaStream_t stream = (cudaStream_t)stream_;
+  if (a->elem != EL_F32 || !scratch || paired_ld(a->K) > (1ll << 29)) return (int)cudaErrorInvalidValue;
+  B2xGemmArgs g = *a;
+  g.a_k_stride = g.b_k_stride = 1;
+  g.a_row_stride = g.b_row_stride = 2 * paired_ld(a->K);
+  g.a_batch_stride = a->M * g.a_row_stride;
+  g.b_batch_stride = a->N * g.b_row_stride;
+  char* b_split = (char*)scratch + (a->batch * g.a_batch_stride * 4 + 1023) / 1024 * 1024;
+  g.a = scratch; g.b = b_split;
+  int rc = launch_split(a, (float*)scratch, (float*)b_split, true, stream);
+  if (rc) return rc;
+  return launch_gemm_tc(&g, epilogue, true, status, stream);
 }

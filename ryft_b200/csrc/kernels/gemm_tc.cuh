@@ -45,6 +45,13 @@ struct TcParams {
   // freed 48 KB double the bulk-store epilogue's staging tiles, so that a warp fills one while the TMA engine still reads the
   // other (with one tile it waited 200-350 cycles per strip for the previous store to have read it).
   int32_t short_k;
+  // f32 operands split into high and low TF32 halves (3xTF32): rows hold [hi | lo], the low half `lo_off` elements behind the
+  // high one.  A stage holds both halves of both operands and a k-step issues hi * hi, hi * lo and lo * hi on it, so every
+  // tile is loaded once for the products it takes part in; with operands laid out as [hi | hi | lo] and [hi | lo | hi] along a
+  // threefold K the high halves were loaded (and written to scratch) twice.  Shared memory's 128 bytes per clock bound this
+  // kernel (128 x 256 tiles, per 32 of K: 192 KB loaded and read instead of 240), SPLIT_NOW.
+  int32_t paired;
+  int32_t lo_off;
   int32_t num_m_tiles, num_n_tiles;
   int64_t num_tiles;
   int32_t k_blocks;
@@ -190,9 +197,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
   pdl_wait();          // everything above touched this SM only
   // stage geometry: the ring is STAGES * STAGE_BYTES either way (tall tiles are only routed to the <256, 4> kernels,
   // whose 4 x 48 KB ring is 3 x 64 KB)
-  const int n_stages = (p.tall || p.short_k) ? 3 : STAGES;
-  const uint32_t a_bytes = p.tall ? 2u * SM::A_BYTES : (uint32_t)SM::A_BYTES;
-  const uint32_t stage_bytes = a_bytes + (uint32_t)SM::B_BYTES;
+  const bool paired = TF32 && p.paired;
+  const int n_stages = (p.tall || p.short_k) ? 3 : (paired ? STAGES / 2 : STAGES);
+  const uint32_t a_bytes = (p.tall || paired) ? 2u * SM::A_BYTES : (uint32_t)SM::A_BYTES;
+  const uint32_t stage_bytes = a_bytes + (paired ? 2u : 1u) * (uint32_t)SM::B_BYTES;
 
 
   if (warp == 0) {
@@ -237,6 +245,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
           mbar_expect_tx(full, stage_bytes);
           const uint32_t sa = smem_base + stage * stage_bytes, sb = sa + a_bytes;
           const int k0 = kb * BK;
+          if (paired) {
+            tma_load_3d(sa + SM::A_BYTES, &tmA, full, p.lo_off + k0, m0, b);
+            tma_load_3d(sb + SM::B_BYTES, &tmB, full, p.lo_off + k0, n0, b);
+          }
           if (!p.a_mn_major) tma_load_3d(sa, &tmA, full, k0, m0, b);
           else if (p.a_mn_4d) tma_load_4d(sa, &tmA, full, 0, k0, m0 / CHUNK, b);
           else {
@@ -301,6 +313,10 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; k++) {
             umma_ss<TF32>(d_tmem, a_desc0 + (uint64_t)(k * a_adv), b_desc0 + (uint64_t)(k * b_adv), p.idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            if (paired) {
+              umma_ss<TF32>(d_tmem, a_desc0 + (uint64_t)(k * a_adv), b_desc0 + (uint64_t)(k * b_adv) + (uint64_t)(SM::B_BYTES >> 4), p.idesc, 1u);
+              umma_ss<TF32>(d_tmem, a_desc0 + (uint64_t)(k * a_adv) + (uint64_t)(SM::A_BYTES >> 4), b_desc0 + (uint64_t)(k * b_adv), p.idesc, 1u);
+            }
             // tall tiles: rows 128..255 of the stage's A (16 KB further in either layout) against the same B sub-tile
             if (p.tall) umma_ss<TF32>(d_tmem + (uint32_t)BN, a_desc0 + (uint64_t)(k * a_adv) + (uint64_t)(SM::A_BYTES >> 4), b_desc0 + (uint64_t)(k * b_adv), p.idesc,
                                       (kb > 0 || k > 0) ? 1u : 0u);

@@ -112,19 +112,8 @@ PJRT_Error* run_plan(PJRT_LoadedExecutable* le, int local_index, int replica, co
         if (s.wide) {
           rc = b2x_launch_wide_gemm(&ga, (uint8_t)s.w_out_dtype, bind(s.w_out), cs);
         } else if (s.g_tensor_core) {
-          if (s.g_split_f32) {
-            // A' = [hi | hi | lo], B' = [hi | lo | hi]: K-major rows of 3K floats in scratch
-            float* a_split = (float*)bind(s.scratch);
-            size_t a_elems = (size_t)(s.gB * s.gM * 3 * s.gK);
-            float* b_split = a_split + ((a_elems + 255) / 256) * 256;
-            rc = b2x_launch_split_f32(&ga, a_split, b_split, cs);
-            if (rc) return kernel_error(rc, s);
-            ga.a = a_split; ga.b = b_split;
-            ga.K = 3 * s.gK;
-            ga.a_k_stride = 1; ga.a_row_stride = ga.K; ga.a_batch_stride = s.gM * ga.K;
-            ga.b_k_stride = 1; ga.b_row_stride = ga.K; ga.b_batch_stride = s.gN * ga.K;
-          }
-          rc = b2x_launch_gemm_tc(&ga, &prog, dev->status_dev, cs);
+          rc = s.g_split_f32 ? b2x_launch_gemm_f32(&ga, &prog, bind(s.scratch), dev->status_dev, cs)
+                             : b2x_launch_gemm_tc(&ga, &prog, dev->status_dev, cs);
         } else {
           rc = b2x_launch_gemm_simt(&ga, &prog, s.vm.vec, cs);
         }

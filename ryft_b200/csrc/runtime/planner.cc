@@ -1458,9 +1458,9 @@ void Planner::emit_dot(const Op& op) {
   s.g_tensor_core = opt_.allow_tensor_core && tc_dtype && M >= 128 && N >= 64 && N % 8 == 0 && s.gK >= 32 &&
                     tc_operand_ok(s.ga, M) && tc_operand_ok(s.gb, N);
   if (s.g_tensor_core && in_dt == DType::F32) {
-    // three TF32 products over hi/lo splits: A' = [Ahi | Ahi | Alo], B' = [Bhi | Blo | Bhi] along K, held in scratch
+    // three TF32 products over hi/lo splits held in scratch
     s.g_split_f32 = true;
-    s.scratch_bytes = (s.gB * M * 3 * s.gK + s.gB * N * 3 * s.gK) * 4 + 2048;
+    s.scratch_bytes = b2x_gemm_f32_scratch_bytes(s.gB, M, N, s.gK);
     s.scratch = new_temp(s.scratch_bytes);
   }
 
