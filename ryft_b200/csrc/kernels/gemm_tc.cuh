@@ -49,7 +49,7 @@ struct TcParams {
   // high one.  A stage holds both halves of both operands and a k-step issues hi * hi, hi * lo and lo * hi on it, so every
   // tile is loaded once for the products it takes part in; with operands laid out as [hi | hi | lo] and [hi | lo | hi] along a
   // threefold K the high halves were loaded (and written to scratch) twice.  Shared memory's 128 bytes per clock bound this
-  // kernel (128 x 256 tiles, per 32 of K: 192 KB loaded and read instead of 240), SPLIT_NOW.
+  // kernel (128 x 256 tiles, per 32 of K: 192 KB loaded and read instead of 240), 4096 x 2048 x 4096 429 -> 389 us, 1024^3 35.6 -> 28.7.
   int32_t paired;
   int32_t lo_off;
   int32_t num_m_tiles, num_n_tiles;
