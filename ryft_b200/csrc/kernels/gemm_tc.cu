@@ -35,31 +35,47 @@ int32_t* sched_slot(cudaStream_t stream) {
 
 // ---- f32 -> hi/lo TF32 split for the 3xTF32 scheme ------------------------------------------------------------------
 // out rows are K-major: sel 0 -> [hi | hi | lo] and sel 1 -> [hi | lo | hi] with 3K elements, sel 2 -> [hi | lo] with 2 ld
-// elements, each half padded with zeros from K to ld.  One launch splits both
-// operands: a CTA takes 32 x 32 (row, k) tiles of either.  A source that is contiguous along k is read and written
-// with lane = k; any other source is read with lane = row and turned through shared memory, so that the writes are
-// contiguous along k as well.
+// elements, each half padded with zeros from K to ld.  One launch splits both operands, in tiles of 32 x 128.  A source that
+// is contiguous along k is read along k, 16 bytes per lane where its rows allow; any other source is read along the rows and
+// turned through shared memory.  Either way 16 values per thread are in flight before the first is needed, and the halves
+// leave as 16-byte pieces of rows.  HBM-bound: 4 bytes in, 8 out per element (sel 2).  2 x [2048, 4096] contracted over the
+// first dimension: 64 us with 32 x 32 tiles and 4 bytes per access; the whole product 389 -> 364 us.
 // Elements of one half of a paired row: whole k-blocks, so that none straddles the two halves.
 static int64_t paired_ld(int64_t K) { return (K + 31) / 32 * 32; }
 struct SplitSide {
   const float* src; float* dst;
   int64_t rows, K, ld, pitch, sb, sr, sk;   // ld: elements of a half, pitch: of an output row
   int64_t tiles_r, tiles_k, n_tiles;
-  int sel;
+  int sel, wide;                            // wide: rows of the source can be read, rows of the result written, 16 bytes at a time
 };
-__device__ __forceinline__ void split_write(float* o, int64_t K, int64_t k, float x, int sel) {
+__device__ __forceinline__ float2 split_value(float x) {
   const float hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-  const float lo = __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u);
-  o[k] = hi;
-  if (sel == 2) { o[K + k] = lo; return; }
-  o[K + k] = sel == 0 ? hi : lo;
-  o[2 * K + k] = sel == 0 ? lo : hi;
+  return make_float2(hi, __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u));
+}
+__device__ __forceinline__ void split_write(const SplitSide& S, float* o, int64_t k, const float (&x)[4]) {
+  float2 v[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) v[j] = split_value(x[j]);
+  if (S.wide) {
+    const float4 hi = make_float4(v[0].x, v[1].x, v[2].x, v[3].x), lo = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+    *(float4*)(o + k) = hi;
+    *(float4*)(o + S.ld + k) = S.sel == 0 ? hi : lo;
+    if (S.sel != 2) *(float4*)(o + 2 * S.ld + k) = S.sel == 0 ? lo : hi;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (k + j < S.ld) {
+        o[k + j] = v[j].x;
+        o[S.ld + k + j] = S.sel == 0 ? v[j].x : v[j].y;
+        if (S.sel != 2) o[2 * S.ld + k + j] = S.sel == 0 ? v[j].y : v[j].x;
+      }
+  }
 }
 __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B) {
-  __shared__ float tile[32][33];
+  __shared__ float tile[32][129];
   pdl_trigger();
   pdl_wait();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t total = A.n_tiles + B.n_tiles;
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
     const bool second = t >= A.n_tiles;
@@ -68,31 +84,57 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
     const int64_t tk = u % S.tiles_k; u /= S.tiles_k;
     const int64_t tr = u % S.tiles_r;
     const int64_t b = u / S.tiles_r;
-    const int64_t r0 = tr * 32, k0 = tk * 32;
     const float* src = S.src + b * S.sb;
     float* dst = S.dst + b * S.rows * S.pitch;
     if (S.sk == 1) {
-      const int64_t k = k0 + tx;
+      // 32 rows x 128 k: a warp per row, four rows each
+      const int64_t r0 = tr * 32 + warp, k = tk * 128 + lane * 4;
+      float x[4][4];
 #pragma unroll
-      for (int i = ty; i < 32; i += 8) {
-        const int64_t r = r0 + i;
-        if (r < S.rows && k < S.ld) split_write(dst + r * S.pitch, S.ld, k, k < S.K ? __ldg(src + r * S.sr + k) : 0.0f, S.sel);
+      for (int i = 0; i < 4; i++) {
+        const int64_t r = r0 + i * 8;
+        const float* p = src + r * S.sr + k;
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[i][j] = 0.f;
+        if (r < S.rows) {
+          if (S.wide && k + 3 < S.K) {
+            const float4 f = __ldg((const float4*)p);
+            x[i][0] = f.x; x[i][1] = f.y; x[i][2] = f.z; x[i][3] = f.w;
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) if (k + j < S.K) x[i][j] = __ldg(p + j);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int64_t r = r0 + i * 8;
+        if (r < S.rows && k < S.ld) split_write(S, dst + r * S.pitch, k, x[i]);
       }
     } else {
-      const int64_t r_in = r0 + tx;
+      // 128 rows x 32 k: read along the rows, four k lines per warp; written along k, eight lanes to a row's 128 bytes
+      const int64_t r0 = tr * 128, k0 = tk * 32;
+      float x[4][4];
 #pragma unroll
-      for (int i = ty; i < 32; i += 8) {
-        const int64_t k = k0 + i;
-        tile[i][tx] = (r_in < S.rows && k < S.K) ? __ldg(src + r_in * S.sr + k * S.sk) : 0.0f;
-      }
-      __syncthreads();
-      const int64_t k = k0 + tx;
+      for (int i = 0; i < 4; i++)
 #pragma unroll
-      for (int i = ty; i < 32; i += 8) {
-        const int64_t r = r0 + i;
-        if (r < S.rows && k < S.ld) split_write(dst + r * S.pitch, S.ld, k, tile[tx][i], S.sel);
-      }
+        for (int j = 0; j < 4; j++) {
+          const int64_t k = k0 + warp * 4 + i, r = r0 + j * 32 + lane;
+          x[i][j] = (r < S.rows && k < S.K) ? __ldg(src + r * S.sr + k * S.sk) : 0.0f;
+        }
+      __syncthreads();        // the previous tile has been written out
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) tile[warp * 4 + i][j * 32 + lane] = x[i][j];
       __syncthreads();
+      const int kk = (lane & 7) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int rr = i * 32 + warp * 4 + (lane >> 3);
+        const float y[4] = {tile[kk][rr], tile[kk + 1][rr], tile[kk + 2][rr], tile[kk + 3][rr]};
+        if (r0 + rr < S.rows && k0 + kk < S.ld) split_write(S, dst + (r0 + rr) * S.pitch, k0 + kk, y);
+      }
     }
   }
 }
@@ -106,7 +148,9 @@ static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bo
     SplitSide s{};
     s.src = (const float*)src; s.dst = dst; s.rows = rows; s.K = a->K; s.sb = sb; s.sr = sr; s.sk = sk; s.sel = sel;
     s.ld = paired ? paired_ld(a->K) : a->K; s.pitch = paired ? 2 * s.ld : 3 * a->K;
-    s.tiles_r = (rows + 31) / 32; s.tiles_k = (a->K + 31) / 32; s.n_tiles = a->batch * s.tiles_r * s.tiles_k;
+    const int tr = sk == 1 ? 32 : 128, tk = sk == 1 ? 128 : 32;
+    s.tiles_r = (rows + tr - 1) / tr; s.tiles_k = (s.ld + tk - 1) / tk; s.n_tiles = a->batch * s.tiles_r * s.tiles_k;
+    s.wide = (uintptr_t)dst % 16 == 0 && s.ld % 4 == 0 && s.pitch % 4 == 0 && (sk != 1 || ((uintptr_t)src % 16 == 0 && sr % 4 == 0 && (a->batch == 1 || sb % 4 == 0)));
     return s;
   };
   const SplitSide A = side(a->a, a_split, a->M, a->a_batch_stride, a->a_row_stride, a->a_k_stride, paired ? 2 : 0);
