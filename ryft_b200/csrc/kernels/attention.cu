@@ -930,6 +930,8 @@ extern "C" int b2x_launch_attention(const B2xAttentionArgs* a, int32_t* status, 
   // unmasked ones of 128-wide heads with tiles of 16 and more key blocks.  Device times, persistent / one-tile:
   //   causal, 128 wide: 29 heads x 512 20.9 / 12.3 us, 8 x 4096 84 / 45, 16 x 4096 84 / 86, 32 x 4096 158 / 172, 128 x 4096 592 / 661
   //   unmasked: 32 x 4096 x 128 313 / 283, 64 x 2048 x 128 171 / 164, 32 x 2048 x 64 76 / 82, 24 x 1000 x 64 26.5 / 26.7
+  // These were measured side by side before the issuing threads were elected.  With that, causal 16 x 4096 80 / 78, 32 x 4096
+  // 144 / 159, 128 x 4096 552 / 610, unmasked 32 x 2048 x 64 74 / 78, and the one-tile form 43 on 8 x 4096 and 258 on unmasked 32 x 4096 x 128.
   // B2X_ATTENTION_KERNEL=tile / persistent selects one of them.
   const char* form = getenv("B2X_ATTENTION_KERNEL");
   const int64_t tiles = (a->Sq + AT_M - 1) / AT_M * a->BH;
