@@ -925,17 +925,24 @@ extern "C" int b2x_launch_attention(const B2xAttentionArgs* a, int32_t* status, 
   if (a->BH <= 0 || a->Sq <= 0 || a->Sk <= 0) return (int)cudaErrorInvalidValue;
   if (((uintptr_t)a->q & 15) || ((uintptr_t)a->k & 15) || ((uintptr_t)a->v & 15) || ((uintptr_t)a->o & 15)) return (int)cudaErrorInvalidValue;
   // Which form: the persistent two-worker kernel hides a tile's start-up and write-out behind the other worker, the
-  // one-tile-per-CTA kernel puts both halves of the SM on one tile and runs a little faster per key block.  So the latter
-  // takes problems that would leave a worker at most one tile (two per SM), where it halves the longest tile's time, and
-  // unmasked ones of 128-wide heads with tiles of 16 and more key blocks.  Device times, persistent / one-tile:
-  //   causal, 128 wide: 29 heads x 512 20.9 / 12.3 us, 8 x 4096 84 / 45, 16 x 4096 84 / 86, 32 x 4096 158 / 172, 128 x 4096 592 / 661
-  //   unmasked: 32 x 4096 x 128 313 / 283, 64 x 2048 x 128 171 / 164, 32 x 2048 x 64 76 / 82, 24 x 1000 x 64 26.5 / 26.7
-  // These were measured side by side before the issuing threads were elected.  With that, causal 16 x 4096 80 / 78, 32 x 4096
-  // 144 / 159, 128 x 4096 552 / 610, unmasked 32 x 2048 x 64 74 / 78, and the one-tile form 43 on 8 x 4096 and 258 on unmasked 32 x 4096 x 128.
+  // one-tile-per-CTA kernel puts both halves of the SM on one tile and halves the time of a launch whose tiles do not come
+  // to two per SM; it also runs a little faster per key block of long unmasked 128-wide heads.  Device times in us,
+  // one-tile / persistent (sequence x width, heads -> tiles):
+  //   up to one tile per SM          512 x 64, 29 -> 116: causal 8.4 / 14.4, unmasked 8.3 / 14.4; 4096 x 128, 4 -> 128: 39 / 73, 39 / 77
+  //   one to two tiles, causal       1000 x 64, 24 -> 192: 12.9 / 22.1; 4096 x 128, 8 -> 256: 39 / 75; 1000 x 128, 37 -> 296: 20.7 / 25.7
+  //   one to two tiles, unmasked     1000 x 64, 24 -> 192: 22.9 / 23.7; 1920 x 64, 16 -> 240: 37.1 / 37.2; 512 x 64, 64 -> 256: 15.6 / 15.1;
+  //                                  1000 x 128, 37 -> 296: 28.0 / 27.5 (each worker has a tile of the same length: no difference)
+  //   causal, more                   4096 x 128, 16 -> 512: 77.8 / 75.4, 32 -> 1024: 160 / 145, 128 -> 4096: 610 / 566; 512 x 64, 80 -> 320: 17.9 / 15.4
+  //   unmasked, 128 wide, more       2048, 24 -> 384: 61 / 79, 64 -> 1024: 150 / 155; 4096, 16 -> 512: 135 / 146, 32 -> 1024: 261 / 289;
+  //                                  below 16 key blocks the other way round: 512, 128 -> 512: 36.1 / 31.6, 1000, 128 -> 1024: 98 / 90
+  //   unmasked, 64 wide, more        2048, 32 -> 512: 75 / 73, 128 -> 2048: 270 / 243
+  // The two keep their running maxima over different blocks, so the weights are rounded to bf16 against different maxima:
+  // results differ by 2.5e-3 while the error against 64 bits of the one-tile form is 0 to 4 % below the other's.  Where
+  // neither is faster the persistent form stays.
   // B2X_ATTENTION_KERNEL=tile / persistent selects one of them.
   const char* form = getenv("B2X_ATTENTION_KERNEL");
   const int64_t tiles = (a->Sq + AT_M - 1) / AT_M * a->BH;
-  bool one_tile = tiles <= 2 * kNumSms || (!a->causal && a->D == 128 && a->Sk > 15 * AT_N);
+  bool one_tile = tiles <= (a->causal ? 2 : 1) * kNumSms || (!a->causal && a->D == 128 && a->Sk > 15 * AT_N);
   if (form && (form[0] == 't' || form[0] == 'p')) one_tile = form[0] == 't';
   if (!one_tile && (a->D == 128 || a->D == 64)) {
     const int rc = a->D == 128 ? launch_attention_pw<128>(a, status, stream) : launch_attention_pw<64>(a, status, stream);

@@ -100,6 +100,24 @@ def test_cuda_core_product_with_epilogue(client, M, K, N):
     check_program(client, text, ins, f"epilogue {M}x{K}x{N}", f32_tol=1e-6)
 
 
+# which of the two attention kernels takes a problem: they round the weights against different maxima, so their results tell
+# them apart.  Up to one tile per SM (148) and one above, causal up to two per SM and one above, unmasked long 128-wide heads
+@pytest.mark.parametrize("B,H,S,D,causal,form", [(1, 74, 200, 64, False, "tile"), (1, 75, 200, 64, False, "persistent"), (2, 12, 1000, 64, False, "persistent"),
+                                                 (1, 148, 200, 64, False, "persistent"), (1, 148, 200, 64, True, "tile"), (1, 149, 200, 64, True, "persistent"),
+                                                 (1, 19, 1000, 128, False, "persistent"), (1, 19, 1930, 128, False, "tile"), (1, 40, 1930, 64, False, "persistent")])
+def test_attention_form(client, monkeypatch, B, H, S, D, causal, form):
+    from helpers import run_gpu
+    text, ins = configs.c3_program(B, H, S, D, causal=causal), configs.c3_inputs(B, H, S, D)
+    monkeypatch.delenv("B2X_ATTENTION_KERNEL", raising=False)
+    (chosen,) = run_gpu(client, text, ins)
+    got = {}
+    for f in ("tile", "persistent"):
+        monkeypatch.setenv("B2X_ATTENTION_KERNEL", f)
+        (got[f],) = run_gpu(client, text, ins)
+    assert not np.array_equal(got["tile"].view(np.int16), got["persistent"].view(np.int16))
+    assert np.array_equal(chosen.view(np.int16), got[form].view(np.int16))
+
+
 # the order in which query tiles are dealt out: a last group of fewer heads, one head per group, both kernel forms on either
 # side of the rule between them; rows and heads that are missed or computed twice show as wrong rows
 @pytest.mark.parametrize("B,H,S,D,causal", [(1, 5, 300, 64, True), (1, 37, 1100, 64, True), (1, 19, 2100, 128, True), (2, 10, 2050, 128, False)])
