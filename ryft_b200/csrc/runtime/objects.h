@@ -15,6 +15,7 @@
 
 #include "../../../include/b2x_pjrt_c_api.h"
 #include "plan.h"
+#include "stream_mark.h"
 
 struct PJRT_Error {
   PJRT_Error_Code code;
@@ -34,37 +35,6 @@ PJRT_Error* cuda_error(cudaError_t e, const char* what);
     PJRT_Error* _err = (expr);                \
     if (_err) return _err;                    \
   } while (0)
-}  // namespace b2x
-
-namespace b2x {
-// A point in a stream's work: an event recorded once and never again, shared by everything that has to know when the
-// stream has got there (the outputs of an execution, the views it read, its completion).  One event per execution instead
-// of one per output, argument and completion: creating, recording and destroying them was a third of the execute call.
-struct StreamMark {
-  cudaEvent_t ev = nullptr;
-  cudaStream_t stream = nullptr;
-  ~StreamMark() { if (ev) cudaEventDestroy(ev); }
-};
-using MarkRef = std::shared_ptr<StreamMark>;
-// Records a mark behind the work that `stream` holds now (the stream's device must be current).  The mark exists also when
-// recording failed: whoever waits for it is then told.
-inline cudaError_t mark_stream(cudaStream_t stream, MarkRef* out) {
-  MarkRef m = std::make_shared<StreamMark>();
-  m->stream = stream;
-  cudaError_t e = cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventRecord(m->ev, stream);
-  *out = std::move(m);
-  return e;
-}
-// Makes `stream` wait for a mark; nothing to do when the mark lies on the stream itself.
-inline cudaError_t wait_mark(cudaStream_t stream, const MarkRef& m) {
-  return m && m->stream != stream ? cudaStreamWaitEvent(stream, m->ev, 0) : cudaSuccess;
-}
-// Remembers a reader.  A later mark of the same stream covers the earlier one, so the list holds one per stream.
-inline void add_mark(std::vector<MarkRef>* marks, MarkRef m) {
-  for (auto& o : *marks) if (o->stream == m->stream) { o = std::move(m); return; }
-  marks->push_back(std::move(m));
-}
 }  // namespace b2x
 
 // Host-visible completion object.  Thread-safe; callbacks run exactly once, on the thread that completes the event
@@ -110,6 +80,7 @@ struct PJRT_Device {
   bool addressable = false;
   int cuda_ordinal = -1;
   cudaStream_t compute = nullptr, h2d = nullptr, d2h = nullptr, comm = nullptr;
+  b2x::MarkClock marks;   // of the four streams
   PJRT_Memory* memory = nullptr;
   std::vector<PJRT_Memory*> memories;
   int32_t* status_host = nullptr;  // pinned, mapped: kernels write a non-zero code when a bounded wait expires

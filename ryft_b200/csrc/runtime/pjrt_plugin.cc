@@ -603,7 +603,7 @@ static PJRT_Error* Client_BufferFromHostBuffer(PJRT_Client_BufferFromHostBuffer_
   }
   cudaError_t e = cudaSuccess;
   if (b->bytes) e = cudaMemcpyAsync(b->ptr, src, b->bytes, cudaMemcpyHostToDevice, dev->h2d);
-  if (e == cudaSuccess) e = mark_stream(dev->h2d, &b->ready);
+  if (e == cudaSuccess) e = mark_stream(&dev->marks, dev->h2d, &b->ready);
   if (e != cudaSuccess) { release_buffer_memory(b); delete b; return cuda_error(e, "host to device copy"); }
   PJRT_Event* done = new PJRT_Event();
   const bool must_finish_now = a->host_buffer_semantics == PJRT_HostBufferSemantics_kImmutableOnlyDuringCall || !dense;
@@ -657,7 +657,7 @@ static PJRT_Error* Client_CreateViewOfDeviceBuffer(PJRT_Client_CreateViewOfDevic
   }
   if (a->stream) {  // work already queued on the producer's stream must finish before this buffer is read
     cudaSetDevice(dev->cuda_ordinal);
-    mark_stream((cudaStream_t)a->stream, &b->ready);
+    mark_stream(nullptr, (cudaStream_t)a->stream, &b->ready);
   }
   a->buffer = b;
   return nullptr;
@@ -758,7 +758,7 @@ static PJRT_Error* copy_to_host(PJRT_Buffer* b, void* dst, size_t offset, size_t
   }
   if (size) B2X_CUDA(cudaMemcpyAsync(staging ? staging : dst, (const char*)b->ptr + offset, size, cudaMemcpyDeviceToHost, d->d2h));
   MarkRef copied;
-  B2X_CUDA(mark_stream(d->d2h, &copied));
+  B2X_CUDA(mark_stream(&d->marks, d->d2h, &copied));
   add_mark(&b->pending_reads, copied);   // freeing the buffer waits for the copy
   PJRT_Event* pe = new PJRT_Event();
   PJRT_Device* dev = d;
@@ -806,7 +806,7 @@ static PJRT_Error* copy_to_device_impl(PJRT_Buffer* b, PJRT_Device* dst_dev, PJR
     if (dst_dev == b->device) e = cudaMemcpyAsync(nb->ptr, b->ptr, b->bytes, cudaMemcpyDeviceToDevice, dst_dev->compute);
     else e = cudaMemcpyPeerAsync(nb->ptr, dst_dev->cuda_ordinal, b->ptr, b->device->cuda_ordinal, b->bytes, dst_dev->compute);
   }
-  if (e == cudaSuccess) e = mark_stream(dst_dev->compute, &nb->ready);
+  if (e == cudaSuccess) e = mark_stream(&dst_dev->marks, dst_dev->compute, &nb->ready);
   if (e != cudaSuccess) { release_buffer_memory(nb); delete nb; return cuda_error(e, "device to device copy"); }
   // the source must outlive the copy: remember the read on the source buffer
   add_mark(&b->pending_reads, nb->ready);
@@ -1234,8 +1234,8 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
     // everything this execution has enqueued: on the compute stream, and behind its detached collectives
     MarkRef computed, done;
     if (!failed) {
-      mark_stream(dev->compute, &computed);
-      if (done_stream == dev->compute) done = computed; else mark_stream(done_stream, &done);
+      mark_stream(&dev->marks, dev->compute, &computed);
+      if (done_stream == dev->compute) done = computed; else mark_stream(&dev->marks, done_stream, &done);
     }
     for (size_t o = 0; o < n_outs; o++) {
       PJRT_Buffer* ob = o < L.out_bufs.size() ? L.out_bufs[o] : nullptr;
@@ -1413,7 +1413,7 @@ static void finish_definition(PJRT_Buffer* b, PJRT_Error_Code code, const std::s
   PJRT_Device* dev = b->device;
   cudaSetDevice(dev->cuda_ordinal);
   if (code == PJRT_Error_Code_OK) {
-    mark_stream(dev->h2d, &b->ready);
+    mark_stream(&dev->marks, dev->h2d, &b->ready);
   } else {
     b->err_code = code;
     b->err_msg = msg;
@@ -1505,7 +1505,7 @@ static PJRT_Error* transfer_into(PJRT_AsyncHostToDeviceTransferManager* tm, int 
   if (size) B2X_CUDA(cudaMemcpyAsync((char*)b->ptr + offset, data, (size_t)size, cudaMemcpyHostToDevice, dev->h2d));
   PJRT_Event* ev = new PJRT_Event();
   MarkRef copied;
-  mark_stream(dev->h2d, &copied);
+  mark_stream(&dev->marks, dev->h2d, &copied);
   tm->client->post({copied, dev->cuda_ordinal, ev, nullptr});
   *done = ev;
   if (last) { s.finished = true; finish_definition(b, PJRT_Error_Code_OK, ""); }

@@ -1,0 +1,66 @@
+// Points in a stream's work, and who has to wait for them.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <memory>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+namespace b2x {
+// An event recorded once and never again, shared by everything that has to know when the stream has got there (the outputs
+// of an execution, the views it read, its completion).  One event per execution instead of one per output, argument and
+// completion: creating, recording and destroying them was a third of the execute call.
+struct StreamMark {
+  cudaEvent_t ev = nullptr;
+  cudaStream_t stream = nullptr;
+  uint64_t order = 0;             // of two marks on one of the plugin's streams, the later one has the larger number
+  StreamMark() = default;
+  StreamMark(const StreamMark&) = delete;
+  StreamMark& operator=(const StreamMark&) = delete;
+  ~StreamMark() { if (ev) cudaEventDestroy(ev); }
+};
+using MarkRef = std::shared_ptr<StreamMark>;
+
+// Numbers the marks of a device's streams in the order in which they are recorded.
+struct MarkClock {
+  std::mutex mu;
+  uint64_t last = 0;
+};
+
+// Records a mark behind the work that `stream` holds now (the stream's device must be current); `clock` is the device's for
+// one of the plugin's streams and null for a caller's.  The mark exists also when recording failed: whoever waits for it is
+// then told.
+inline cudaError_t mark_stream(MarkClock* clock, cudaStream_t stream, MarkRef* out) {
+  MarkRef m = std::make_shared<StreamMark>();
+  m->stream = stream;
+  cudaError_t e = cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming);
+  if (clock) {
+    std::lock_guard<std::mutex> lk(clock->mu);   // number and record together: two threads may be marking one stream
+    m->order = ++clock->last;
+    if (e == cudaSuccess) e = cudaEventRecord(m->ev, stream);
+  } else if (e == cudaSuccess) {
+    e = cudaEventRecord(m->ev, stream);
+  }
+  *out = std::move(m);
+  return e;
+}
+
+// Makes `stream` wait for a mark; nothing to do when the mark lies on the stream itself.
+inline cudaError_t wait_mark(cudaStream_t stream, const MarkRef& m) {
+  if (!m || m->stream == stream) return cudaSuccess;
+  return cudaStreamWaitEvent(stream, m->ev, 0);
+}
+
+// Remembers a reader.  The later of two marks of one stream covers the earlier one, whichever is added first (executions
+// on two threads record their marks in one order and may add them in the other), so the list holds one per stream.
+inline void add_mark(std::vector<MarkRef>* marks, MarkRef m) {
+  for (auto& o : *marks)
+    if (o->stream == m->stream) {
+      if (o->order < m->order) o = std::move(m);
+      return;
+    }
+  marks->push_back(std::move(m));
+}
+}  // namespace b2x

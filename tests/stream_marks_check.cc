@@ -1,0 +1,80 @@
+// Host checks of runtime/stream_mark.h over a CUDA runtime of a few lines: a stream is a count of the work enqueued on it, an
+// event the count at which it was recorded.  Exits non-zero at the first check that fails.
+#include <atomic>
+#include <cstdio>
+#include <cstdlib>
+#include <thread>
+
+#include "stream_mark.h"
+
+struct CUstream_st { std::atomic<long> work{0}; };
+struct CUevent_st { long at = -1; };
+
+static std::atomic<int> events{0};
+
+extern "C" {
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  events++;
+  *e = new CUevent_st();
+  return cudaSuccess;
+}
+cudaError_t cudaEventDestroy(cudaEvent_t e) { events--; delete e; return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  e->at = s->work.load();
+  return cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+}
+
+#define CHECK(c)                                                          \
+  do {                                                                    \
+    if (!(c)) { fprintf(stderr, "line %d: %s\n", __LINE__, #c); exit(1); } \
+  } while (0)
+
+using namespace b2x;
+
+int main() {
+  {  // two executions record A, then B, and add B, then A: the list has to keep waiting for B
+    MarkClock clock;
+    CUstream_st s;
+    MarkRef a, b;
+    s.work = 1;
+    CHECK(mark_stream(&clock, &s, &a) == cudaSuccess);
+    s.work = 2;
+    CHECK(mark_stream(&clock, &s, &b) == cudaSuccess);
+    std::vector<MarkRef> list;
+    add_mark(&list, b);
+    add_mark(&list, a);
+    CHECK(list.size() == 1 && list[0]->ev->at == 2);
+    list.clear();
+    add_mark(&list, a);
+    add_mark(&list, b);
+    CHECK(list.size() == 1 && list[0]->ev->at == 2);
+  }
+  {  // the same with threads: enqueue, mark, add
+    MarkClock clock;
+    CUstream_st s, other;
+    std::mutex list_mu;
+    std::vector<MarkRef> list;
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 8; t++)
+      threads.emplace_back([&] {
+        for (int i = 0; i < 2000; i++) {
+          const long mine = ++s.work;
+          MarkRef m;
+          CHECK(mark_stream(&clock, &s, &m) == cudaSuccess && m->ev->at >= mine);
+          std::lock_guard<std::mutex> lk(list_mu);
+          add_mark(&list, m);
+          CHECK(list.size() == 1 && list[0]->ev->at >= mine);
+        }
+      });
+    for (auto& t : threads) t.join();
+    CHECK(list[0]->ev->at == 16000);
+    MarkRef m;
+    CHECK(mark_stream(&clock, &other, &m) == cudaSuccess);
+    add_mark(&list, m);
+    CHECK(list.size() == 2);
+  }
+  CHECK(events == 0);
+  return 0;
+}
