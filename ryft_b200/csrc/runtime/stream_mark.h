@@ -14,6 +14,9 @@ namespace b2x {
 // completion: creating, recording and destroying them was a third of the execute call.
 struct StreamMark {
   cudaEvent_t ev = nullptr;
+  // The plugin's own stream that the mark lies on; null on a caller's.  Only the plugin's streams are told apart by their
+  // handles: they live as long as the client, while a caller's handle can stand for another stream in another thread
+  // (cudaStreamPerThread) or, once the stream has been destroyed, for a new one.
   cudaStream_t stream = nullptr;
   uint64_t order = 0;             // of two marks on one of the plugin's streams, the later one has the larger number
   StreamMark() = default;
@@ -34,10 +37,10 @@ struct MarkClock {
 // then told.
 inline cudaError_t mark_stream(MarkClock* clock, cudaStream_t stream, MarkRef* out) {
   MarkRef m = std::make_shared<StreamMark>();
-  m->stream = stream;
   cudaError_t e = cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming);
   if (clock) {
     std::lock_guard<std::mutex> lk(clock->mu);   // number and record together: two threads may be marking one stream
+    m->stream = stream;
     m->order = ++clock->last;
     if (e == cudaSuccess) e = cudaEventRecord(m->ev, stream);
   } else if (e == cudaSuccess) {
@@ -49,18 +52,19 @@ inline cudaError_t mark_stream(MarkClock* clock, cudaStream_t stream, MarkRef* o
 
 // Makes `stream` wait for a mark; nothing to do when the mark lies on the stream itself.
 inline cudaError_t wait_mark(cudaStream_t stream, const MarkRef& m) {
-  if (!m || m->stream == stream) return cudaSuccess;
+  if (!m || (m->stream && m->stream == stream)) return cudaSuccess;
   return cudaStreamWaitEvent(stream, m->ev, 0);
 }
 
 // Remembers a reader.  The later of two marks of one stream covers the earlier one, whichever is added first (executions
 // on two threads record their marks in one order and may add them in the other), so the list holds one per stream.
 inline void add_mark(std::vector<MarkRef>* marks, MarkRef m) {
-  for (auto& o : *marks)
-    if (o->stream == m->stream) {
-      if (o->order < m->order) o = std::move(m);
-      return;
-    }
+  if (m->stream)
+    for (auto& o : *marks)
+      if (o->stream == m->stream) {
+        if (o->order < m->order) o = std::move(m);
+        return;
+      }
   marks->push_back(std::move(m));
 }
 }  // namespace b2x

@@ -11,6 +11,7 @@ struct CUstream_st { std::atomic<long> work{0}; };
 struct CUevent_st { long at = -1; };
 
 static std::atomic<int> events{0};
+static int waits = 0;
 
 extern "C" {
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
@@ -23,7 +24,7 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
   e->at = s->work.load();
   return cudaSuccess;
 }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t e, unsigned) { waits += e != nullptr; return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
 }
 
 #define CHECK(c)                                                          \
@@ -73,6 +74,24 @@ int main() {
     MarkRef m;
     CHECK(mark_stream(&clock, &other, &m) == cudaSuccess);
     add_mark(&list, m);
+    CHECK(list.size() == 2);
+  }
+  {  // the wait on the mark's own stream is left out only for the plugin's streams
+    MarkClock clock;
+    CUstream_st s, t;
+    MarkRef own, foreign;
+    CHECK(mark_stream(&clock, &s, &own) == cudaSuccess && mark_stream(nullptr, &t, &foreign) == cudaSuccess);
+    waits = 0;
+    CHECK(wait_mark(&s, own) == cudaSuccess && waits == 0);
+    CHECK(wait_mark(&t, own) == cudaSuccess && waits == 1);
+    CHECK(wait_mark(&s, foreign) == cudaSuccess && waits == 2);
+    CHECK(wait_mark(&t, foreign) == cudaSuccess && waits == 3);
+    CHECK(wait_mark(&s, nullptr) == cudaSuccess && waits == 3);
+    std::vector<MarkRef> list;
+    add_mark(&list, foreign);
+    MarkRef again;
+    CHECK(mark_stream(nullptr, &t, &again) == cudaSuccess);
+    add_mark(&list, again);
     CHECK(list.size() == 2);
   }
   CHECK(events == 0);
