@@ -657,7 +657,8 @@ static PJRT_Error* Client_CreateViewOfDeviceBuffer(PJRT_Client_CreateViewOfDevic
   }
   if (a->stream) {  // work already queued on the producer's stream must finish before this buffer is read
     cudaSetDevice(dev->cuda_ordinal);
-    mark_stream(nullptr, (cudaStream_t)a->stream, &b->ready);
+    const cudaError_t e = mark_stream(nullptr, (cudaStream_t)a->stream, &b->ready);
+    if (e != cudaSuccess) { delete b; return cuda_error(e, "marking the producer's stream"); }
   }
   a->buffer = b;
   return nullptr;
@@ -1219,11 +1220,10 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
     PJRT_Device* dev = le->addressable[locals[k]];
     PerLaunch& L = launches[k];
     cudaSetDevice(dev->cuda_ordinal);
-    const bool failed = L.err != nullptr;
     // Collectives that the compute stream does not wait for still belong to this execution: its outputs and its
     // completion event are recorded on the communication stream, behind everything the compute stream has queued.
     cudaStream_t done_stream = dev->compute;
-    if (!failed && le->core->plans[0].has_detached_collectives) {
+    if (!L.err && le->core->plans[0].has_detached_collectives) {
       cudaEvent_t join;
       cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
       cudaEventRecord(join, dev->compute);
@@ -1233,10 +1233,13 @@ static PJRT_Error* LoadedExecutable_Execute(PJRT_LoadedExecutable_Execute_Args* 
     }
     // everything this execution has enqueued: on the compute stream, and behind its detached collectives
     MarkRef computed, done;
-    if (!failed) {
-      mark_stream(&dev->marks, dev->compute, &computed);
-      if (done_stream == dev->compute) done = computed; else mark_stream(&dev->marks, done_stream, &done);
+    if (!L.err) {
+      cudaError_t e = mark_stream(&dev->marks, dev->compute, &computed);
+      if (done_stream == dev->compute) done = computed;
+      else if (e == cudaSuccess) e = mark_stream(&dev->marks, done_stream, &done);
+      if (e != cudaSuccess) L.err = cuda_error(e, "marking the end of an execution");
     }
+    const bool failed = L.err != nullptr;
     for (size_t o = 0; o < n_outs; o++) {
       PJRT_Buffer* ob = o < L.out_bufs.size() ? L.out_bufs[o] : nullptr;
       if (!ob) {
@@ -1407,14 +1410,16 @@ struct PJRT_AsyncHostToDeviceTransferManager {
 };
 
 // Completes a buffer's pending definition: `code` OK means its contents are whatever the transfer stream holds now.
-static void finish_definition(PJRT_Buffer* b, PJRT_Error_Code code, const std::string& msg) {
+static void finish_definition(PJRT_Buffer* b, PJRT_Error_Code code, std::string msg) {
   std::shared_ptr<b2x_Definition> d = b->pending;
   if (!d) return;
   PJRT_Device* dev = b->device;
   cudaSetDevice(dev->cuda_ordinal);
   if (code == PJRT_Error_Code_OK) {
-    mark_stream(&dev->marks, dev->h2d, &b->ready);
-  } else {
+    const cudaError_t e = mark_stream(&dev->marks, dev->h2d, &b->ready);
+    if (e != cudaSuccess) { code = PJRT_Error_Code_INTERNAL; msg = std::string("host to device copy: ") + cudaGetErrorString(e); }
+  }
+  if (code != PJRT_Error_Code_OK) {
     b->err_code = code;
     b->err_msg = msg;
   }
@@ -1503,9 +1508,9 @@ static PJRT_Error* transfer_into(PJRT_AsyncHostToDeviceTransferManager* tm, int 
   PJRT_Device* dev = tm->device;
   B2X_CUDA(cudaSetDevice(dev->cuda_ordinal));
   if (size) B2X_CUDA(cudaMemcpyAsync((char*)b->ptr + offset, data, (size_t)size, cudaMemcpyHostToDevice, dev->h2d));
-  PJRT_Event* ev = new PJRT_Event();
   MarkRef copied;
-  mark_stream(&dev->marks, dev->h2d, &copied);
+  B2X_CUDA(mark_stream(&dev->marks, dev->h2d, &copied));
+  PJRT_Event* ev = new PJRT_Event();
   tm->client->post({copied, dev->cuda_ordinal, ev, nullptr});
   *done = ev;
   if (last) { s.finished = true; finish_definition(b, PJRT_Error_Code_OK, ""); }

@@ -24,7 +24,7 @@ struct StreamMark {
   StreamMark& operator=(const StreamMark&) = delete;
   ~StreamMark() { if (ev) cudaEventDestroy(ev); }
 };
-using MarkRef = std::shared_ptr<StreamMark>;
+using MarkRef = std::shared_ptr<StreamMark>;   // null: nothing to wait for
 
 // Numbers the marks of a device's streams in the order in which they are recorded.
 struct MarkClock {
@@ -33,21 +33,27 @@ struct MarkClock {
 };
 
 // Records a mark behind the work that `stream` holds now (the stream's device must be current); `clock` is the device's for
-// one of the plugin's streams and null for a caller's.  The mark exists also when recording failed: whoever waits for it is
-// then told.
+// one of the plugin's streams and null for a caller's.  Where no event can be had, the work is waited for right here and the
+// mark is null; an error means that the work itself has failed or cannot be waited for.
 inline cudaError_t mark_stream(MarkClock* clock, cudaStream_t stream, MarkRef* out) {
+  out->reset();
   MarkRef m = std::make_shared<StreamMark>();
   cudaError_t e = cudaEventCreateWithFlags(&m->ev, cudaEventDisableTiming);
-  if (clock) {
+  if (e != cudaSuccess) m->ev = nullptr;
+  else if (clock) {
     std::lock_guard<std::mutex> lk(clock->mu);   // number and record together: two threads may be marking one stream
     m->stream = stream;
     m->order = ++clock->last;
-    if (e == cudaSuccess) e = cudaEventRecord(m->ev, stream);
-  } else if (e == cudaSuccess) {
+    e = cudaEventRecord(m->ev, stream);
+  } else {
     e = cudaEventRecord(m->ev, stream);
   }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cudaStreamSynchronize(stream);
+  }
   *out = std::move(m);
-  return e;
+  return cudaSuccess;
 }
 
 // Makes `stream` wait for a mark; nothing to do when the mark lies on the stream itself.
@@ -59,6 +65,7 @@ inline cudaError_t wait_mark(cudaStream_t stream, const MarkRef& m) {
 // Remembers a reader.  The later of two marks of one stream covers the earlier one, whichever is added first (executions
 // on two threads record their marks in one order and may add them in the other), so the list holds one per stream.
 inline void add_mark(std::vector<MarkRef>* marks, MarkRef m) {
+  if (!m) return;
   if (m->stream)
     for (auto& o : *marks)
       if (o->stream == m->stream) {

@@ -7,24 +7,29 @@
 
 #include "stream_mark.h"
 
-struct CUstream_st { std::atomic<long> work{0}; };
+struct CUstream_st { std::atomic<long> work{0}; long synchronised = -1; };
 struct CUevent_st { long at = -1; };
 
+static bool create_fails = false, record_fails = false;
 static std::atomic<int> events{0};
 static int waits = 0;
 
 extern "C" {
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
+  if (create_fails) return cudaErrorMemoryAllocation;
   events++;
   *e = new CUevent_st();
   return cudaSuccess;
 }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { events--; delete e; return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  if (record_fails) return cudaErrorLaunchFailure;
   e->at = s->work.load();
   return cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t e, unsigned) { waits += e != nullptr; return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { s->synchronised = s->work.load(); return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
 }
 
 #define CHECK(c)                                                          \
@@ -93,6 +98,20 @@ int main() {
     CHECK(mark_stream(nullptr, &t, &again) == cudaSuccess);
     add_mark(&list, again);
     CHECK(list.size() == 2);
+  }
+  for (bool* failure : {&create_fails, &record_fails}) {  // no event: the work is waited for, and an earlier mark is not given up
+    MarkClock clock;
+    CUstream_st s;
+    MarkRef before, m;
+    s.work = 3;
+    CHECK(mark_stream(&clock, &s, &before) == cudaSuccess);
+    std::vector<MarkRef> list{before};
+    s.work = 4;
+    *failure = true;
+    CHECK(mark_stream(&clock, &s, &m) == cudaSuccess && !m && s.synchronised == 4);
+    *failure = false;
+    add_mark(&list, m);
+    CHECK(list.size() == 1 && list[0] == before);
   }
   CHECK(events == 0);
   return 0;

@@ -1,4 +1,5 @@
-"""Marks in a stream's work (runtime/stream_mark.h): which of two marks a buffer keeps and which waits are left out.  The header is compiled for the host against a stand-in for the CUDA runtime."""
+"""Marks in a stream's work (runtime/stream_mark.h): which of two marks a buffer keeps, which waits are left out, what happens
+when no event can be had.  The header is compiled for the host against a stand-in for the CUDA runtime."""
 import os
 import shutil
 import subprocess
