@@ -256,10 +256,20 @@ static int tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bool pai
 }
 }  // namespace b2x
 
-extern "C" int b2x_gemm_tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t out[12]) {
-  using namespace b2x;
+namespace b2x {
+// The product that the tensor cores make of an f32 problem once its operands lie in scratch as rows of [hi | lo]: K stays.
+static B2xGemmArgs paired_problem(const B2xGemmArgs& a) {
+  B2xGemmArgs g = a;
+  g.a_k_stride = g.b_k_stride = 1;
+  g.a_row_stride = g.b_row_stride = 2 * paired_ld(a.K);
+  g.a_batch_stride = a.M * g.a_row_stride;
+  g.b_batch_stride = a.N * g.b_row_stride;
+  return g;
+}
+
+static int report_route(const B2xGemmArgs& a, const B2xVmProgram* epilogue, bool paired, int32_t out[12]) {
   TcRoute r;
-  int rc = tc_route(a, epilogue, false, &r);
+  int rc = tc_route(&a, epilogue, paired, &r);
   if (rc) return rc;
   out[0] = r.BN; out[1] = r.static_id; out[2] = r.p.epi_groups;
   out[3] = (r.static_id && r.p.transposed && tc_static_stores(r.static_id) >= 2) ? 1 : 0;
@@ -267,8 +277,18 @@ extern "C" int b2x_gemm_tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilo
   out[8] = r.static_id ? tc_static_stores(r.static_id) : 0;
   out[9] = (int32_t)(r.p.num_tiles < kNumSms ? r.p.num_tiles : kNumSms);
   out[10] = r.p.tall ? 2 * TC_BM : TC_BM;
-  out[11] = 0;
+  out[11] = r.p.paired;
   return 0;
+}
+}  // namespace b2x
+
+extern "C" int b2x_gemm_tc_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t out[12]) {
+  return b2x::report_route(*a, epilogue, false, out);
+}
+
+extern "C" int b2x_gemm_f32_route(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t out[12]) {
+  if (a->elem != EL_F32) return (int)cudaErrorInvalidValue;
+  return b2x::report_route(b2x::paired_problem(*a), epilogue, true, out);
 }
 
 namespace b2x {
@@ -335,11 +355,7 @@ extern "C" int b2x_launch_gemm_f32(const B2xGemmArgs* a, const B2xVmProgram* epi
   using namespace b2x;
   cudaStream_t stream = (cudaStream_t)stream_;
   if (a->elem != EL_F32 || !scratch || paired_ld(a->K) > (1ll << 29)) return (int)cudaErrorInvalidValue;
-  B2xGemmArgs g = *a;
-  g.a_k_stride = g.b_k_stride = 1;
-  g.a_row_stride = g.b_row_stride = 2 * paired_ld(a->K);
-  g.a_batch_stride = a->M * g.a_row_stride;
-  g.b_batch_stride = a->N * g.b_row_stride;
+  B2xGemmArgs g = paired_problem(*a);
   char* b_split = (char*)scratch + (a->batch * g.a_batch_stride * 4 + 1023) / 1024 * 1024;
   g.a = scratch; g.b = b_split;
   int rc = launch_split(a, (float*)scratch, (float*)b_split, true, stream);

@@ -112,7 +112,8 @@ extern "C" __attribute__((visibility("default"))) int b2x_plan_signatures(const 
 #include "../../../include/b2x_kernels.h"
 
 // Lists, one line per tensor-core GEMM step of the module's plan, the kernel variant the launcher will pick:
-//   label|M|N|K|batch|BN|static id|epilogue groups|transposed|group_m|m tiles|n tiles|k blocks|stores|ctas
+//   label|M|N|K|batch|BN|static id|epilogue groups|transposed|group_m|m tiles|n tiles|k blocks|stores|ctas|tile rows|paired
+// K counts what the tensor cores multiply per result: three products for each k of an f32 problem (paired = 1).
 extern "C" __attribute__((visibility("default"))) int b2x_plan_routes(const char* mlir, size_t mlir_size, int num_replicas, char* out, size_t out_cap,
                                                                        size_t* out_size) {
   std::string text;
@@ -128,15 +129,10 @@ extern "C" __attribute__((visibility("default"))) int b2x_plan_routes(const char
       ga.batch = s.gB; ga.M = s.gM; ga.N = s.gN; ga.K = s.gK;
       ga.a_batch_stride = s.ga.batch_stride; ga.a_row_stride = s.ga.row_stride; ga.a_k_stride = s.ga.k_stride;
       ga.b_batch_stride = s.gb.batch_stride; ga.b_row_stride = s.gb.row_stride; ga.b_k_stride = s.gb.k_stride;
-      if (s.g_split_f32) {
-        ga.K = 3 * s.gK;
-        ga.a_k_stride = 1; ga.a_row_stride = ga.K; ga.a_batch_stride = s.gM * ga.K;
-        ga.b_k_stride = 1; ga.b_row_stride = ga.K; ga.b_batch_stride = s.gN * ga.K;
-      }
       int32_t r[12] = {};
-      int rc = b2x_gemm_tc_route(&ga, &s.vm.prog, r);
-      text += s.label + "|" + std::to_string(s.gM) + "|" + std::to_string(s.gN) + "|" + std::to_string(ga.K) + "|" + std::to_string(s.gB);
-      for (int i = 0; i < 11; i++) text += "|" + std::to_string(rc ? -1 : r[i]);
+      int rc = s.g_split_f32 ? b2x_gemm_f32_route(&ga, &s.vm.prog, r) : b2x_gemm_tc_route(&ga, &s.vm.prog, r);
+      text += s.label + "|" + std::to_string(s.gM) + "|" + std::to_string(s.gN) + "|" + std::to_string((s.g_split_f32 ? 3 : 1) * s.gK) + "|" + std::to_string(s.gB);
+      for (int i = 0; i < 12; i++) text += "|" + std::to_string(rc ? -1 : r[i]);
       text += "\n";
     }
   } catch (const b2x::CompileError& e) {

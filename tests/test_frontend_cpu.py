@@ -241,3 +241,20 @@ def test_benchmark_programs_take_specialised_gemm_variants():
     assert (r2["bn"], r2["epi_groups"], r2["k_blocks"], r2["stores"], r2["tile_rows"]) == (256, 1, 2, 1, 128) and r2["static_id"]
     (r1,) = ryft_b200.plan_routes(configs.c1_program())
     assert r1["K"] == 3 * 768 and r1["static_id"]
+
+
+def test_routes_of_f32_products_are_those_of_the_paired_kernel():
+    """f32 operands: a k-block is 32 of the problem's K (both halves of both operands), and a raster group's slab of A, 32 MiB,
+    counts both halves, whatever the operands' layout."""
+    (r1,) = ryft_b200.plan_routes(configs.c1_program())
+    assert (r1["paired"], r1["k_blocks"], r1["bn"], r1["m_tiles"], r1["n_tiles"]) == (1, 768 // 32, 64, 4, 8)
+    for lc in (0, 1):
+        b = Builder()
+        x = b.arg([2048, 4096] if lc == 0 else [4096, 2048], "f32"); y = b.arg([2048, 4096], "f32")
+        (r,) = ryft_b200.plan_routes(b.build(b.dot_general(x, y, ([], []), ([lc], [0]))))
+        assert (r["paired"], r["k_blocks"], r["epi_groups"], r["group_m"]) == (1, 2048 // 32, 2, (32 << 20) // (128 * 2048 * 4 * 2))
+    b = Builder()
+    x = b.arg([300, 68], "f32"); y = b.arg([68, 72], "f32")
+    (r,) = ryft_b200.plan_routes(b.build(b.dot_general(x, y, ([], []), ([1], [0]))))
+    assert (r["paired"], r["k_blocks"], r["epi_groups"]) == (1, 3, 2)
+    assert all(r["paired"] == 0 for r in ryft_b200.plan_routes(configs.c4_program()))
