@@ -412,7 +412,7 @@ static int direct_kind(const B2xVmProgram& P, const ReduceKArgs& K, int vec) {
 
 // Column reduction.  A cluster of CL CTAs owns 128 or 64 adjacent columns (32 without vectors) of one (outer, split) piece;
 // its rows are dealt to the CTAs and their thread rows in turn, so that at any moment the whole cluster sweeps one band
-// of the tensor.  blockDim = (BX, RY) with BX * RY = 256; thread (bx, ry) owns V adjacent columns.  The thread rows meet
+// of the tensor.  blockDim = (BX, RY) with BX * RY between 32 and 256; thread (bx, ry) owns V adjacent columns.  The thread rows meet
 // in shared memory, the CTAs of the cluster through distributed shared memory, always in the same order.
 // HBM-bound; what decides is how many bytes are in flight, i.e. how many CTAs there are.  [8192, 4096] f32 -> [4096]:
 // 3557 us with one CTA per 2048 columns and row split (8 CTAs, one interpreted row in flight per thread) and a second
@@ -533,11 +533,15 @@ static int launch_cols(const B2xVmProgram& P, const ReduceKArgs& K, const B2xVmP
   if (DIRECT != 0 && V > 1 && K.A * K.S * ((bvecs + bx_max - 1) / bx_max) * 8 < (int64_t)kNumSms * 4) bx_max /= 2;
   int bx = 1;
   while (bx < bx_max && bx < bvecs) bx <<= 1;
-  const int ry = 256 / bx;
+  const int64_t rows = K.chunk < K.R ? K.chunk : K.R;
+  // no more thread rows than rows, down to a warp: the others would only take part in the barriers that combine them, and the
+  // smaller CTAs leave the SM room for more pieces ([100000, 8, 3] over the middle, 64 -> 8 thread rows: 264 -> 39 us, 474 -> 82
+  // with a product in front; [4096, 16, 16] 26.3 -> 8.8 us)
+  int ry = 256 / bx;
+  while (bx * ry > 32 && ry / 2 >= rows) ry /= 2;
   const int n_bblocks = (int)((bvecs + bx - 1) / bx);
   const int64_t work = K.A * K.S * (int64_t)n_bblocks;
   // as many CTAs per cluster as it takes to have four per SM, while each thread still has several rows
-  const int64_t rows = K.chunk < K.R ? K.chunk : K.R;
   int CL = 1;
   while (CL < 8 && work * CL < (int64_t)kNumSms * 4 && rows >= (int64_t)ry * CL * 8) CL *= 2;
   int64_t clusters = work;

@@ -30,6 +30,21 @@ def test_column_reduction(client, shape, dtype, body):
     check_program(client, text, [v], f"{body} {dtype} {shape}", f32_tol=1e-6)
 
 
+# pieces of fewer rows than a CTA has thread rows: one row, a power of two, one more, columns with and without vectors, in every
+# element kind, with a program in front of the reduction and a consumer behind it
+@pytest.mark.parametrize("shape", [(1000, 1, 5), (3000, 8, 3), (77, 9, 24), (300, 16, 16), (5, 33, 136), (1, 2, 2)])
+@pytest.mark.parametrize("dtype,body,fused", [("f32", "add", False), ("f32", "add", True), ("bf16", "maximum", False), ("i32", "add", False), ("f32", "minimum", True)])
+def test_column_reduction_of_few_rows(client, shape, dtype, body, fused):
+    b = Builder()
+    x = b.arg(shape, dtype)
+    init = b.constant({"add": 0 if dtype == "i32" else 0.0, "maximum": float("-inf"), "minimum": float("inf")}[body], [], dtype)
+    r = b.reduce(b.multiply(x, x) if fused else x, init, body, [1])
+    text = b.build(b.convert(b.multiply(r, b.splat(0.5, r)), "bf16") if fused else r)
+    g = np.random.default_rng(8)
+    v = g.integers(-1000, 1000, size=shape).astype(np.int32) if dtype == "i32" else g.standard_normal(shape, dtype=np.float32).astype(configs.np_dtype(dtype))
+    check_program(client, text, [v], f"{body} {dtype} {shape}", f32_tol=1e-6)
+
+
 def softmax_program(shape, out_dtype="f32", extra=False):
     lead = list(range(len(shape) - 1))
     b = Builder()
