@@ -25,6 +25,13 @@ __device__ __forceinline__ float sm_max(float a, float b) {
   return r;
 }
 
+// The sum of N values from v[AT] on, added in pairs.
+template <int AT, int N, int E>
+__device__ __forceinline__ float sm_tree_sum(const float (&v)[E]) {
+  if constexpr (N == 1) return v[AT];
+  else return sm_tree_sum<AT, N / 2>(v) + sm_tree_sum<AT + N / 2, N / 2>(v);
+}
+
 // T threads per row (32: eight rows per CTA), E elements per thread in pieces of V adjacent ones, OUT: B2xElem of the result.
 template <int T, int E, int V, int OUT>
 __global__ void __launch_bounds__(T == 32 ? 256 : T) k_softmax_rows(const float* __restrict__ x, char* __restrict__ out, int64_t rows, int n) {
@@ -61,23 +68,29 @@ __global__ void __launch_bounds__(T == 32 ? 256 : T) k_softmax_rows(const float*
 #pragma unroll
       for (int w = 1; w < T / 32; w++) m = sm_max(m, smem[0][w]);
     }
-    float s = 0.f;
+    // a piece's four values are added in pairs, and pieces go to two partial sums in turn (single values to eight): at most six
+    // additions in a row instead of E
+    constexpr int PARTS = V == 4 ? 2 : 8;
+    float part[PARTS];
+#pragma unroll
+    for (int i = 0; i < PARTS; i++) part[i] = 0.f;
 #pragma unroll
     for (int i = 0; i < P; i++) {
       if ((i * T + tid) * V < n) {
+        float piece[V];
 #pragma unroll
-        for (int j = 0; j < V; j++) { v[i * V + j] = expf(v[i * V + j] - m); s += v[i * V + j]; }
+        for (int j = 0; j < V; j++) piece[j] = v[i * V + j] = expf(v[i * V + j] - m);
+        part[i % PARTS] += sm_tree_sum<0, V>(piece);
       }
     }
+    float s = sm_tree_sum<0, PARTS>(part);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
     if constexpr (T > 32) {
       // smem[1] is read again only behind the next row's first barrier
       if ((tid & 31) == 0) smem[1][tid >> 5] = s;
       __syncthreads();
-      s = smem[1][0];
-#pragma unroll
-      for (int w = 1; w < T / 32; w++) s += smem[1][w];
+      s = sm_tree_sum<0, T / 32>(smem[1]);
     }
     constexpr int ES = OUT == EL_F32 ? 4 : 2;
     char* dst = out + row * n * ES;

@@ -76,6 +76,23 @@ def test_row_softmax(client, shape, out_dtype):
     check_program(client, text, [x], f"softmax {out_dtype} {shape}", f32_tol=1e-6)
 
 
+# the row sums are no less exact than those of the two reductions and two elementwise passes that the kernel stands for, in each
+# of its width classes (the maximum, the exponentials and the quotients are the same values)
+@pytest.mark.parametrize("n", [512, 1024, 2048, 4096, 8192, 16384])
+def test_row_softmax_is_as_exact_as_the_chain(client, monkeypatch, n):
+    from helpers import run_gpu
+    rows = 1 << 23 >> (n.bit_length() - 1)
+    x = np.random.default_rng(13).standard_normal((rows, n), dtype=np.float32) * np.float32(3)
+    e = np.exp(x.astype(np.float64) - x.max(axis=1, keepdims=True))
+    want = e / e.sum(axis=1, keepdims=True)
+    error = {}
+    for fused in ("1", "0"):
+        monkeypatch.setenv("B2X_FUSED_SOFTMAX", fused)
+        (got,) = run_gpu(client, softmax_program((rows, n)), [x])
+        error[fused] = np.linalg.norm(got - want) / np.linalg.norm(want)
+    assert error["1"] <= error["0"], error
+
+
 def test_row_softmax_of_a_value_that_is_also_returned(client):
     shape = (6, 200)
     check_program(client, softmax_program(shape, extra=True), [np.random.default_rng(4).standard_normal(shape, dtype=np.float32)], "softmax, operand returned", f32_tol=1e-6)
