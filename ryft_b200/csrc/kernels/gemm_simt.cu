@@ -94,8 +94,7 @@ __global__ void __launch_bounds__(256) k_gemm_simt(const __grid_constant__ GemmK
   constexpr int A_WORDS = 16 * (BM + 4), B_WORDS = 16 * (BN + 4);
   constexpr int RING = 2 * (A_WORDS + B_WORDS), TILE = BM * BN;
   __shared__ __align__(16) uint32_t sm[RING > TILE ? RING : TILE];
-  pdl_trigger();
-  pdl_wait();
+  pdl_trigger();     // nothing to wait for: the operands come through the read-only path, so this kernel is launched in its turn
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int rank = G.CL > 1 ? (int)(blockIdx.x % (unsigned)G.CL) : 0;
   const unsigned tile = blockIdx.x / (unsigned)G.CL;
@@ -220,13 +219,11 @@ static int launch_simt(GemmK G, const B2xVmProgram& P, int vec, cudaStream_t str
   cfg.gridDim = dim3((unsigned)(tiles * CL), 1, (unsigned)(G.batch > 1024 ? 1024 : G.batch));
   cfg.blockDim = dim3(256);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2]{};
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = (unsigned)CL; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = CL > 1 ? 2 : 1;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)CL; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = CL > 1 ? 1 : 0;
   const int V = simt_plain_store(P, G) ? 0 : ((vec >= 4 && G.N % 4 == 0) ? 4 : 1);
   if (V == 0) { G.plain_out = (char*)P.tensors[0].ptr; G.plain_elem = P.tensors[0].elem; }
   cudaError_t e;

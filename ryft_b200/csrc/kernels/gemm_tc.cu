@@ -71,7 +71,7 @@ __device__ __forceinline__ void split_write(const SplitSide& S, float* o, int64_
       }
   }
 }
-__global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B) {
+__global__ void __launch_bounds__(256, 4) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B) {
   __shared__ float tile[32][129];
   pdl_trigger();
   pdl_wait();
@@ -98,11 +98,11 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
         for (int j = 0; j < 4; j++) x[i][j] = 0.f;
         if (r < S.rows) {
           if (S.wide && k + 3 < S.K) {
-            const float4 f = __ldg((const float4*)p);
+            const float4 f = ld_global((const float4*)p);
             x[i][0] = f.x; x[i][1] = f.y; x[i][2] = f.z; x[i][3] = f.w;
           } else {
 #pragma unroll
-            for (int j = 0; j < 4; j++) if (k + j < S.K) x[i][j] = __ldg(p + j);
+            for (int j = 0; j < 4; j++) if (k + j < S.K) x[i][j] = ld_global(p + j);
           }
         }
       }
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_split_f32(const __grid_constant__ Split
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const int64_t k = k0 + warp * 4 + i, r = r0 + j * 32 + lane;
-          x[i][j] = (r < S.rows && k < S.K) ? __ldg(src + r * S.sr + k * S.sk) : 0.0f;
+          x[i][j] = (r < S.rows && k < S.K) ? ld_global(src + r * S.sr + k * S.sk) : 0.0f;
         }
       __syncthreads();        // the previous tile has been written out
 #pragma unroll

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256, ID != 0 ? 4 : 1) k_reduce_rows(const __gr
 // tickets and the same fold as k_reduce_rows; ES = bytes per element (4: f32, 2: bf16), SQ = square each element first,
 // MC = 1 sum / 2 maximum (NaN-propagating).
 template <int ES, bool SQ, int MC>
-__global__ void __launch_bounds__(256) k_reduce_rows_direct(const char* __restrict__ base, const __grid_constant__ ReduceKArgs K,
+__global__ void __launch_bounds__(256) k_reduce_rows_direct(const char* base, const __grid_constant__ ReduceKArgs K,
                                                             const __grid_constant__ B2xVmProgram Q) {
   __shared__ uint32_t smem[8];
   __shared__ int s_last;
@@ -363,16 +363,16 @@ __global__ void __launch_bounds__(256) k_reduce_rows_direct(const char* __restri
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const uint4* p = (const uint4*)(row + (r + u * STEP) * ES);
-        lo[u] = __ldg(p);
-        if constexpr (ES == 4) hi[u] = __ldg(p + 1); else hi[u] = make_uint4(0, 0, 0, 0);
+        lo[u] = ld_global(p);
+        if constexpr (ES == 4) hi[u] = ld_global(p + 1); else hi[u] = make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < U; u++) fold8(tot[u], lo[u], hi[u]);
     }
     for (; r < K.R; r += STEP) {
       const uint4* p = (const uint4*)(row + r * ES);
-      uint4 lo = __ldg(p), hi = make_uint4(0, 0, 0, 0);
-      if constexpr (ES == 4) hi = __ldg(p + 1);
+      uint4 lo = ld_global(p), hi = make_uint4(0, 0, 0, 0);
+      if constexpr (ES == 4) hi = ld_global(p + 1);
       fold8(tot[0], lo, hi);
     }
     uint32_t total = red_combine_t<MC>(red_combine_t<MC>(f2u(tot[0]), f2u(tot[1]), K.monoid, K.cls), red_combine_t<MC>(f2u(tot[2]), f2u(tot[3]), K.monoid, K.cls),
@@ -418,10 +418,11 @@ static int direct_kind(const B2xVmProgram& P, const ReduceKArgs& K, int vec) {
 // 3557 us with one CTA per 2048 columns and row split (8 CTAs, one interpreted row in flight per thread) and a second
 // launch for the four splits; 64 column blocks x 8 CTAs with eight 16-byte loads in flight per thread: 27.0 us (5.0 TB/s) on the device.
 // DIRECT: the prologue is the dense tensor itself, f32 (4) or bf16 (2), and the loop is plain loads and arithmetic
-// (direct_cols); 0: the prologue program.  MC: see red_combine_t.
+// (direct_cols); 0: the prologue program.  MC: see red_combine_t.  The vector forms are held to the 64 registers of four CTAs per
+// SM: left alone, the compiler takes 72 for bf16 ([8192, 4096] 19.4 us, 13.9 so) and spills in the f32 loop (27.1 us, 25.6 so).
 template <int V, int DIRECT, int MC>
-__global__ void __launch_bounds__(256) k_reduce_cols(const __grid_constant__ B2xVmProgram P, const __grid_constant__ ReduceKArgs K, const __grid_constant__ B2xVmProgram Q,
-                                                     const char* __restrict__ base, int n_bblocks, int CL) {
+__global__ void __launch_bounds__(256, DIRECT != 0 && V > 1 ? 4 : 0) k_reduce_cols(const __grid_constant__ B2xVmProgram P, const __grid_constant__ ReduceKArgs K,
+                                                                                   const __grid_constant__ B2xVmProgram Q, const char* base, int n_bblocks, int CL) {
   namespace cg = cooperative_groups;
   __shared__ uint32_t smem[256 * V];
   pdl_trigger();

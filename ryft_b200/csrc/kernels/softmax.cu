@@ -34,7 +34,7 @@ __device__ __forceinline__ float sm_tree_sum(const float (&v)[E]) {
 
 // T threads per row (32: eight rows per CTA), E elements per thread in pieces of V adjacent ones, OUT: B2xElem of the result.
 template <int T, int E, int V, int OUT>
-__global__ void __launch_bounds__(T == 32 ? 256 : T) k_softmax_rows(const float* __restrict__ x, char* __restrict__ out, int64_t rows, int n) {
+__global__ void __launch_bounds__(T == 32 ? 256 : T) k_softmax_rows(const float* x, char* out, int64_t rows, int n) {
   __shared__ float smem[2][T / 32];
   constexpr int ROWS = T == 32 ? 8 : 1;
   constexpr int P = E / V;                              // pieces per thread

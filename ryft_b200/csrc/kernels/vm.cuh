@@ -8,6 +8,7 @@
 #include <cuda_fp16.h>
 #include <math_constants.h>
 
+#include "common.cuh"
 #include "vm.h"
 
 namespace b2x {
@@ -41,20 +42,20 @@ __host__ __device__ __forceinline__ int vm_elem_size(uint8_t e) {
 template <int NB>
 __device__ __forceinline__ void vm_ld_bytes(const void* p, uint32_t* raw) {
   if constexpr (NB == 32) {
-    uint4 a = __ldg((const uint4*)p), b = __ldg((const uint4*)p + 1);
+    const uint4 a = ld_global((const uint4*)p), b = ld_global((const uint4*)p + 1);
     raw[0] = a.x; raw[1] = a.y; raw[2] = a.z; raw[3] = a.w; raw[4] = b.x; raw[5] = b.y; raw[6] = b.z; raw[7] = b.w;
   } else if constexpr (NB == 16) {
-    uint4 a = __ldg((const uint4*)p);
+    const uint4 a = ld_global((const uint4*)p);
     raw[0] = a.x; raw[1] = a.y; raw[2] = a.z; raw[3] = a.w;
   } else if constexpr (NB == 8) {
-    uint2 a = __ldg((const uint2*)p);
+    const uint2 a = ld_global((const uint2*)p);
     raw[0] = a.x; raw[1] = a.y;
   } else if constexpr (NB == 4) {
-    raw[0] = __ldg((const uint32_t*)p);
+    raw[0] = ld_global((const uint32_t*)p);
   } else if constexpr (NB == 2) {
-    raw[0] = __ldg((const uint16_t*)p);
+    raw[0] = ld_global((const uint16_t*)p);
   } else {
-    raw[0] = __ldg((const uint8_t*)p);
+    raw[0] = ld_global((const uint8_t*)p);
   }
 }
 // Stores are streaming (evict-first in L2): results are written once, and a kernel's own operands, which the other
