@@ -101,7 +101,8 @@ B2X_API int b2x_launch_split_f32(const B2xGemmArgs* host_args, float* a_split, f
 
 /* f32 dot_general as three TF32 products on the tensor cores: splits both operands (any strides) into scratch, rows of
  * [hi | lo], and multiplies hi*hi + hi*lo + lo*hi from there.  M, N and the epilogue as for b2x_launch_gemm_tc; `scratch`
- * holds b2x_gemm_f32_scratch_bytes(batch, M, N, K) bytes and is 16-byte aligned.  Two kernels. */
+ * holds b2x_gemm_f32_scratch_bytes(batch, M, N, K) bytes and is 16-byte aligned.  Two kernels.  Infinities and NaN in the
+ * operands come out as they do of an f32 sum of products. */
 B2X_API int64_t b2x_gemm_f32_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K);
 B2X_API int b2x_launch_gemm_f32(const B2xGemmArgs* host_args, const B2xVmProgram* host_epilogue, void* scratch, int32_t* status, b2x_stream_t stream);
 

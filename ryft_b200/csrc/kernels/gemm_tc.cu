@@ -48,14 +48,18 @@ struct SplitSide {
   int64_t tiles_r, tiles_k, n_tiles;
   int sel, wide;                            // wide: rows of the source can be read, rows of the result written, 16 bytes at a time
 };
-__device__ __forceinline__ float2 split_value(float x) {
+__device__ __forceinline__ float2 split_value(float x, bool& nonfinite) {
   const float hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
-  return make_float2(hi, __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u));
+  const float lo = __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u);
+  // an infinite value is its high half alone, and so is a NaN, made quiet: its set bits may all lie in the part cut off
+  const bool special = (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u;
+  nonfinite |= special;
+  return special ? make_float2(x + x, 0.f) : make_float2(hi, lo);
 }
-__device__ __forceinline__ void split_write(const SplitSide& S, float* o, int64_t k, const float (&x)[4]) {
+__device__ __forceinline__ void split_write(const SplitSide& S, float* o, int64_t k, const float (&x)[4], bool& nonfinite) {
   float2 v[4];
 #pragma unroll
-  for (int j = 0; j < 4; j++) v[j] = split_value(x[j]);
+  for (int j = 0; j < 4; j++) v[j] = split_value(x[j], nonfinite);
   if (S.wide) {
     const float4 hi = make_float4(v[0].x, v[1].x, v[2].x, v[3].x), lo = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
     *(float4*)(o + k) = hi;
@@ -71,12 +75,13 @@ __device__ __forceinline__ void split_write(const SplitSide& S, float* o, int64_
       }
   }
 }
-__global__ void __launch_bounds__(256, 4) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B) {
+__global__ void __launch_bounds__(256, 4) k_split_f32(const __grid_constant__ SplitSide A, const __grid_constant__ SplitSide B, uint32_t* nonfinite) {
   __shared__ float tile[32][129];
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t total = A.n_tiles + B.n_tiles;
+  bool bad = false;
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
     const bool second = t >= A.n_tiles;
     const SplitSide& S = second ? B : A;
@@ -109,7 +114,7 @@ __global__ void __launch_bounds__(256, 4) k_split_f32(const __grid_constant__ Sp
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int64_t r = r0 + i * 8;
-        if (r < S.rows && k < S.ld) split_write(S, dst + r * S.pitch, k, x[i]);
+        if (r < S.rows && k < S.ld) split_write(S, dst + r * S.pitch, k, x[i], bad);
       }
     } else {
       // 128 rows x 32 k: read along the rows, four k lines per warp; written along k, eight lanes to a row's 128 bytes
@@ -133,16 +138,17 @@ __global__ void __launch_bounds__(256, 4) k_split_f32(const __grid_constant__ Sp
       for (int i = 0; i < 4; i++) {
         const int rr = i * 32 + warp * 4 + (lane >> 3);
         const float y[4] = {tile[kk][rr], tile[kk + 1][rr], tile[kk + 2][rr], tile[kk + 3][rr]};
-        if (r0 + rr < S.rows && k0 + kk < S.ld) split_write(S, dst + (r0 + rr) * S.pitch, k0 + kk, y);
+        if (r0 + rr < S.rows && k0 + kk < S.ld) split_write(S, dst + (r0 + rr) * S.pitch, k0 + kk, y, bad);
       }
     }
   }
+  bad = __syncthreads_or(bad);
+  if (nonfinite && threadIdx.x == 0) nonfinite[blockIdx.x] = bad ? 1u : 0u;
 }
 
-}  // namespace b2x
-
-namespace b2x {
-static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bool paired, cudaStream_t stream) {
+constexpr int kSplitCtas = kNumSms * 8;
+// `nonfinite`: kSplitCtas words, or null; *n_nonfinite (may be null): how many of them are written.
+static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bool paired, uint32_t* nonfinite, int32_t* n_nonfinite, cudaStream_t stream) {
   if (a->elem != EL_F32) return (int)cudaErrorInvalidValue;
   auto side = [&](const void* src, float* dst, int64_t rows, int64_t sb, int64_t sr, int64_t sk, int sel) {
     SplitSide s{};
@@ -156,9 +162,10 @@ static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bo
   const SplitSide A = side(a->a, a_split, a->M, a->a_batch_stride, a->a_row_stride, a->a_k_stride, paired ? 2 : 0);
   const SplitSide B = side(a->b, b_split, a->N, a->b_batch_stride, a->b_row_stride, a->b_k_stride, paired ? 2 : 1);
   int64_t grid = A.n_tiles + B.n_tiles;
-  if (grid > (int64_t)kNumSms * 8) grid = (int64_t)kNumSms * 8;
+  if (grid > kSplitCtas) grid = kSplitCtas;
+  if (n_nonfinite) *n_nonfinite = (int32_t)grid;
   if (grid < 1) return 0;
-  const cudaError_t e = launch_overlapped(k_split_f32, dim3((unsigned)grid), dim3(256), 0, stream, A, B);
+  const cudaError_t e = launch_overlapped(k_split_f32, dim3((unsigned)grid), dim3(256), 0, stream, A, B, nonfinite);
   if (e != cudaSuccess) return (int)e;
   count_launch(1);
   return (int)cudaGetLastError();
@@ -166,7 +173,7 @@ static int launch_split(const B2xGemmArgs* a, float* a_split, float* b_split, bo
 }  // namespace b2x
 
 extern "C" int b2x_launch_split_f32(const B2xGemmArgs* a, float* a_split, float* b_split, b2x_stream_t stream) {
-  return b2x::launch_split(a, a_split, b_split, false, (cudaStream_t)stream);
+  return b2x::launch_split(a, a_split, b_split, false, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 namespace b2x {
@@ -292,7 +299,9 @@ extern "C" int b2x_gemm_f32_route(const B2xGemmArgs* a, const B2xVmProgram* epil
 }
 
 namespace b2x {
-static int launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bool paired, int32_t* status, cudaStream_t stream) {
+// nonfinite, n_nonfinite: see launch_split; for paired operands only
+static int launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bool paired, const uint32_t* nonfinite, int32_t n_nonfinite, int32_t* status,
+                          cudaStream_t stream) {
   TcRoute r;
   int rc = tc_route(a, epilogue, paired, &r);
   if (rc) return rc;
@@ -304,6 +313,10 @@ static int launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bo
   CUtensorMap tmA, tmB;
   bool ok;
   TcParams p = r.p;
+  p.nonfinite = nonfinite;
+  p.n_nonfinite = n_nonfinite;
+  p.split_a = paired ? (const float*)a->a : nullptr;
+  p.split_b = paired ? (const float*)a->b : nullptr;
   // B2X_GEMM_LOADS=3d keeps one load per 128-byte-wide sub-tile of an MN-major operand (for comparison)
   static const bool folded = [] { const char* e = getenv("B2X_GEMM_LOADS"); return !(e && e[0] == '3'); }();
   p.a_mn_4d = p.b_mn_4d = 0;
@@ -343,12 +356,12 @@ static int launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, bo
 }  // namespace b2x
 
 extern "C" int b2x_launch_gemm_tc(const B2xGemmArgs* a, const B2xVmProgram* epilogue, int32_t* status, b2x_stream_t stream) {
-  return b2x::launch_gemm_tc(a, epilogue, false, status, (cudaStream_t)stream);
+  return b2x::launch_gemm_tc(a, epilogue, false, nullptr, 0, status, (cudaStream_t)stream);
 }
 
 extern "C" int64_t b2x_gemm_f32_scratch_bytes(int64_t batch, int64_t M, int64_t N, int64_t K) {
   const int64_t pitch = 2 * b2x::paired_ld(K) * 4;
-  return (batch * M * pitch + 1023) / 1024 * 1024 + batch * N * pitch;
+  return (batch * M * pitch + 1023) / 1024 * 1024 + batch * N * pitch + b2x::kSplitCtas * 4;   // pitch: whole 256 bytes
 }
 
 extern "C" int b2x_launch_gemm_f32(const B2xGemmArgs* a, const B2xVmProgram* epilogue, void* scratch, int32_t* status, b2x_stream_t stream_) {
@@ -358,7 +371,9 @@ extern "C" int b2x_launch_gemm_f32(const B2xGemmArgs* a, const B2xVmProgram* epi
   B2xGemmArgs g = paired_problem(*a);
   char* b_split = (char*)scratch + (a->batch * g.a_batch_stride * 4 + 1023) / 1024 * 1024;
   g.a = scratch; g.b = b_split;
-  int rc = launch_split(a, (float*)scratch, (float*)b_split, true, stream);
+  uint32_t* nonfinite = (uint32_t*)(b_split + a->batch * g.b_batch_stride * 4);
+  int32_t n_nonfinite = 0;
+  int rc = launch_split(a, (float*)scratch, (float*)b_split, true, nonfinite, &n_nonfinite, stream);
   if (rc) return rc;
-  return launch_gemm_tc(&g, epilogue, true, status, stream);
+  return launch_gemm_tc(&g, epilogue, true, nonfinite, n_nonfinite, status, stream);
 }

@@ -49,9 +49,13 @@ struct TcParams {
   // high one.  A stage holds both halves of both operands and a k-step issues hi * hi, hi * lo and lo * hi on it, so every
   // tile is loaded once for the products it takes part in; with operands laid out as [hi | hi | lo] and [hi | lo | hi] along a
   // threefold K the high halves were loaded (and written to scratch) twice.  Shared memory's 128 bytes per clock bound this
-  // kernel (128 x 256 tiles, per 32 of K: 192 KB loaded and read instead of 240), 4096 x 2048 x 4096 429 -> 389 us, 1024^3 35.6 -> 28.7.
+  // kernel (128 x 256 tiles, per 32 of K: 96 KB loaded and 144 read instead of 144 and 144), 4096 x 2048 x 4096 429 -> 389 us, 1024^3 35.6 -> 28.7.
   int32_t paired;
   int32_t lo_off;
+  const float* split_a;   // the operands themselves, [batch, M or N] rows of 2 lo_off (tc_settle)
+  const float* split_b;
+  const uint32_t* nonfinite;   // one word per CTA of the split: whether it has met an infinity or a NaN
+  int32_t n_nonfinite;
   int32_t num_m_tiles, num_n_tiles;
   int64_t num_tiles;
   int32_t k_blocks;
@@ -140,6 +144,75 @@ struct TcSmem {
   static constexpr int BAR_OFFSET = STAGING_OFFSET + STAGING_BYTES;       // barriers, TMEM slot, tile ring: 384 bytes
   static constexpr int TOTAL = BAR_OFFSET + 384 + 1024;                   // + slack for 1024-byte alignment
 };
+
+// Infinite f32 operands.  An infinite x is split into hi = x, lo = 0, so one of the three products of a step is inf * 0 = NaN
+// where the other operand is exact in its high half, although the f32 product is infinite.  A NaN in an accumulator is
+// therefore decided again from the operands: no product of the row is NaN, and all infinite ones have one sign, then the
+// result is that infinity.  Finite operands pay for one test per tile.  A tile of 128 x 256 such results costs a few
+// milliseconds at K = 2048; the other roles' waits allow about a second.
+//
+// Bit i of the result: row i of `rows` holds a NaN (x) or an infinity (y).  The warp walks each row together.
+__device__ __forceinline__ uint2 tc_nonfinite_rows(const float* x, int64_t pitch, int rows, int64_t K) {
+  const int lane = threadIdx.x & 31;
+  uint2 found = make_uint2(0u, 0u);
+  for (int i = 0; i < rows; i++) {
+    bool nan = false, inf = false;
+    for (int64_t k = lane; k < K; k += 32) {
+      const float v = ld_global(x + i * pitch + k);
+      nan |= v != v;
+      inf |= fabsf(v) == CUDART_INF_F;
+    }
+    if (__any_sync(0xffffffffu, nan)) found.x |= 1u << i;
+    if (__any_sync(0xffffffffu, inf)) found.y |= 1u << i;
+  }
+  return found;
+}
+// Decides the accumulators of one warp's 32 rows again, in TMEM, chunks part, part + col_parts, ... of `width` columns: the
+// ones that this warp goes on to read.  a, b: the operands' rows of the tile's first row (of the warp) and column, their low
+// halves lo_off elements further; rows, cols: how many of them there are.
+template <int BN>
+static __device__ __noinline__ void tc_settle(const float* a, const float* b, int64_t K, int lo_off, int rows, int cols, uint32_t tmem, int part, int col_parts, int width) {
+  using namespace sm100;
+  const int lane = threadIdx.x & 31;
+  const int64_t pitch = 2 * (int64_t)lo_off;
+  const uint2 ra = tc_nonfinite_rows(a, pitch, rows, K);
+  for (int col = part * width; col < BN && col < cols; col += (col + 8) % width ? 8 : (col_parts - 1) * width + 8) {
+    const int n = min(8, cols - col);
+    const uint2 rb = tc_nonfinite_rows(b + col * pitch, pitch, n, K);
+    uint32_t c[8];
+    tmem_ld_32x8(tmem + (uint32_t)col, c);
+    tc_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const float mine = __uint_as_float(c[j]);
+      const bool open = j < n && mine != mine && lane < rows && !(((ra.x >> lane) | (rb.x >> j)) & 1u) && (((ra.y >> lane) | (rb.y >> j)) & 1u);
+      for (uint32_t todo = __ballot_sync(0xffffffffu, open); todo; todo &= todo - 1) {
+        const int i = __ffs(todo) - 1;
+        const float* x = a + i * pitch;
+        const float* y = b + (col + j) * pitch;
+        bool nan = false, pos = false, neg = false;      // of the whole row, after each round of 256 products
+        for (int64_t k0 = 0; k0 < K && !nan && !(pos && neg); k0 += 256) {
+#pragma unroll
+          for (int u = 0; u < 8; u++) {
+            const int64_t k = k0 + u * 32 + lane;
+            if (k < K) {
+              const float t = (ld_global(x + k) + ld_global(x + lo_off + k)) * (ld_global(y + k) + ld_global(y + lo_off + k));
+              nan |= t != t;
+              pos |= t == CUDART_INF_F;
+              neg |= t == -CUDART_INF_F;
+            }
+          }
+          nan = __any_sync(0xffffffffu, nan);
+          pos = __any_sync(0xffffffffu, pos);
+          neg = __any_sync(0xffffffffu, neg);
+        }
+        if (lane == i && !nan && pos != neg) c[j] = __float_as_uint(pos ? CUDART_INF_F : -CUDART_INF_F);
+      }
+    }
+    tmem_st_32x8(tmem + (uint32_t)col, c);
+    tc_wait_st();
+  }
+}
 
 template <int BN, int STAGES, bool TF32, int ID>
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -341,6 +414,11 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     bool ok = true;
     uint32_t stg_sel = 0;
     const VmRowPlan rplan = vm_row_plan(epi, (uint32_t)p.N);
+    bool settle = false;
+    if constexpr (TF32) {
+      for (int i = lane; paired && i < p.n_nonfinite; i += 32) settle |= ld_global(p.nonfinite + i) != 0u;
+      settle = __any_sync(0xffffffffu, settle);
+    }
     for (int64_t local = p.tall ? 0 : group; ok; local += p.tall ? 1 : p.epi_groups) {
       const int slot = (int)(local & (RING - 1));
       if (!mbar_wait(bar_sfull + 8 * slot, (uint32_t)((local / RING) & 1), abort_flag, status, 7)) { ok = false; break; }
@@ -355,6 +433,13 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
       tc_fence_after();
       const int64_t row = (int64_t)m0 + quad * 32 + lane;
       const bool row_ok = row < p.M;
+      if constexpr (TF32) {
+        if (settle && m0 + quad * 32 < p.M) {
+          const int64_t row0 = (int64_t)m0 + quad * 32, pitch = 2 * (int64_t)p.lo_off;
+          tc_settle<BN>(p.split_a + ((int64_t)b * p.M + row0) * pitch, p.split_b + ((int64_t)b * p.N + n0) * pitch, p.K, p.lo_off, (int)min((int64_t)32, p.M - row0),
+                        (int)min((int64_t)BN, p.N - n0), tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN), part, col_parts, ID != 0 ? 32 : 8);
+        }
+      }
       if constexpr (tc_transposed_epilogue<ID>()) {
         // Transposed epilogue: the accumulator chunk goes through shared memory so that four adjacent lanes own one
         // row's 32 columns.  Every global access of the program is then contiguous over 4 lanes x 8 elements (128 bytes
