@@ -522,9 +522,20 @@ static int direct_cols(const B2xVmProgram& P, const ReduceKArgs& K) {
   return T.elem == EL_F32 ? 4 : (T.elem == EL_BF16 ? 2 : 0);
 }
 
-// Clusters of 128 columns that cover at least two waves need no row splits on top (and so no second launch): the eight
-// CTAs of a cluster split the rows already.
-static bool cols_covered_by_clusters(int64_t A, int64_t B) { return A * ((B + 127) / 128) * 8 >= 2 * kNumSms - 40; }
+// Whether the clusters of the column blocks (eight CTAs each, which split the rows already) do without row splits on top, and
+// so without the second launch that folds them.  It pays while a thread has few rows and each SM gets a CTA: at most 64 rows
+// and one CTA per SM, or 128 rows and one and a half.  One launch against splits, time of the latter over the former, for f32 / bf16 sums
+// and an interpreted f32 minimum, at 16, 19, 24, 28, 32 blocks of 128 columns:
+//   8192 rows (64 per thread)     f32 1.23 1.38 1.30 1.25 1.27   bf16 1.81 1.50 1.38 1.25 1.25   minimum 0.71 0.97 1.00 1.25 1.28
+//   16384 rows                    f32 1.07 1.27 1.18 1.14 1.14   bf16 1.63 1.32 1.22 1.09 1.08   minimum 0.71 0.79 0.82 1.04 1.06
+//   65536 rows                    f32 0.87 1.19 1.09 1.03 1.02   bf16 1.24 1.13 1.08 0.94 0.94   minimum 0.52 0.69 0.72 0.92 0.95
+// and from 36 blocks on, where the clusters no longer all fit at once, 0.71 to 1.03, 0.97 to 1.03 and 0.54 to 0.76 at 65536 rows.
+static bool cols_covered_by_clusters(int64_t A, int64_t R, int64_t B) {
+  const int64_t ctas = A * ((B + 127) / 128) * 8;
+  const int64_t lanes = B % 4 == 0 ? (B < 128 ? (B + 7) / 8 : 16) : (B < 32 ? B : 32);   // threads side by side in a thread row
+  const int64_t rows = R * lanes / (8 * 256);                                          // of a thread
+  return rows <= 64 ? ctas >= kNumSms : rows <= 128 && ctas >= kNumSms * 3 / 2;
+}
 
 template <int V, int DIRECT, int MC>
 static int launch_cols(const B2xVmProgram& P, const ReduceKArgs& K, const B2xVmProgram& Q, cudaStream_t stream) {
@@ -675,7 +686,7 @@ extern "C" int b2x_reduce_splits(int64_t A, int64_t R, int64_t B) {
 
 extern "C" int b2x_reduce_launches(int64_t A, int64_t R, int64_t B) {
   if (A <= 0 || B <= 0) return 0;
-  return (b2x_reduce_splits(A, R, B) > 1 && R > 0 && B != 1 && !b2x::cols_covered_by_clusters(A, B)) ? 2 : 1;
+  return (b2x_reduce_splits(A, R, B) > 1 && R > 0 && B != 1 && !b2x::cols_covered_by_clusters(A, R, B)) ? 2 : 1;
 }
 
 extern "C" int b2x_launch_reduce(const B2xVmProgram* prologue, const B2xReduceArgs* a, b2x_stream_t stream_) {
@@ -711,7 +722,7 @@ extern "C" int b2x_launch_reduce(const B2xVmProgram* prologue, const B2xReduceAr
   }
   static const B2xVmProgram kNoPost{};
   const B2xVmProgram& Q = a->host_post ? *a->host_post : kNoPost;
-  if (S <= 1 || a->R == 0 || (a->B != 1 && cols_covered_by_clusters(a->A, a->B))) {
+  if (S <= 1 || a->R == 0 || (a->B != 1 && cols_covered_by_clusters(a->A, a->R, a->B))) {
     K.S = 1; K.chunk = a->R > 0 ? a->R : 1; K.out = a->out;
     return launch_one(*prologue, K, Q, vec, stream);
   }

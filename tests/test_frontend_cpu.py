@@ -258,3 +258,14 @@ def test_routes_of_f32_products_are_those_of_the_paired_kernel():
     (r,) = ryft_b200.plan_routes(b.build(b.dot_general(x, y, ([], []), ([1], [0]))))
     assert (r["paired"], r["k_blocks"], r["epi_groups"]) == (1, 3, 2)
     assert all(r["paired"] == 0 for r in ryft_b200.plan_routes(configs.c4_program()))
+
+
+# either side of the lines between one launch and two of a column reduction: one CTA per SM for up to 64 rows per thread, one and
+# a half for up to 128, never beyond; few columns of many outer pieces, where a thread has few rows of long ones
+@pytest.mark.parametrize("A,R,B,launches", [(1, 8192, 2304, 2), (1, 8192, 2305, 2), (1, 8192, 2312, 1), (1, 8192, 3072, 1), (1, 4096, 2432, 1), (1, 16384, 3456, 2), (1, 16384, 3464, 1),
+                                            (1, 65536, 4096, 2), (1, 4095, 64, 1), (32, 65536, 8, 1), (18, 16384, 64, 2), (19, 16384, 64, 1), (1, 1 << 20, 1, 1)])
+def test_launches_of_a_column_reduction(A, R, B, launches):
+    import ctypes as C
+    lib = C.CDLL(str(ryft_b200.KERNELS_PATH))
+    lib.b2x_reduce_launches.argtypes = [C.c_int64] * 3
+    assert lib.b2x_reduce_launches(A, R, B) == launches

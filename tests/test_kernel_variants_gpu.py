@@ -218,3 +218,17 @@ def test_f32_product_of_non_finite_values(client, B, M, K, N, lc, rc, epilogue):
     with np.errstate(invalid="ignore"):
         got = check_program(client, text, ins, f"f32 {B}x{M}x{K}x{N} {lc}{rc}", f32_tol=1e-6 + 1.5e-8 * K)
     assert np.isinf(got[0]).sum() > 100
+
+
+# clustered column reductions: a 16-bit sum over several CTAs, and a consumer that the first CTA of the cluster runs; either side
+# of the rule between one launch and two
+@pytest.mark.parametrize("R,N", [(8192, 520), (4100, 2568), (8192, 2304), (8192, 2312)])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("consumer", [False, True])
+def test_clustered_column_sum(client, R, N, dtype, consumer):
+    b = Builder()
+    x = b.arg([R, N], dtype)
+    r = b.reduce(b.convert(x, "f32") if dtype != "f32" else x, b.constant(0.0, [], "f32"), "add", [0])
+    text = b.build(b.convert(b.multiply(r, b.splat(0.5, r)), "bf16") if consumer else r)
+    v = np.random.default_rng(18).standard_normal((R, N), dtype=np.float32).astype(configs.np_dtype(dtype))
+    check_program(client, text, [v], f"column sum {dtype} {R}x{N}", f32_tol=1e-6)
