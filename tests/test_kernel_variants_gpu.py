@@ -125,8 +125,7 @@ def test_cuda_core_product_with_epilogue(client, M, K, N):
     d = b.dot_general(x, y, ([], []), ([1], [0]), out_dtype="f32")
     s = b.add(d, b.broadcast_in_dim(bias, [1], [M, N]))
     text = b.build(b.tanh(s), b.convert(s, "bf16"))
-    if " simt" not in ryft_b200.plan_dump(text):
-        pytest.skip("the tensor cores take this product")
+    assert " simt" in ryft_b200.plan_dump(text)
     r = np.random.default_rng(10)
     ins = [(r.standard_normal(s, dtype=np.float32) * np.float32(0.2)).astype(BF16) for s in ((M, K), (K, N))] + [r.standard_normal((N,), dtype=np.float32)]
     check_program(client, text, ins, f"epilogue {M}x{K}x{N}", f32_tol=1e-6)
@@ -150,8 +149,8 @@ def test_attention_form(client, monkeypatch, B, H, S, D, causal, form):
     assert np.array_equal(chosen.view(np.int16), got[form].view(np.int16))
 
 
-# the order in which query tiles are dealt out: a last group of fewer heads, one head per group, both kernel forms on either
-# side of the rule between them; rows and heads that are missed or computed twice show as wrong rows
+# the order in which query tiles are dealt out within one group of heads, both kernel forms on either side of the rule between
+# them; rows and heads that are missed or computed twice show as wrong rows
 @pytest.mark.parametrize("B,H,S,D,causal", [(1, 5, 300, 64, True), (1, 37, 1100, 64, True), (1, 19, 2100, 128, True), (2, 10, 2050, 128, False)])
 def test_attention_tile_order(client, B, H, S, D, causal):
     from helpers import run_gpu
@@ -232,3 +231,173 @@ def test_clustered_column_sum(client, R, N, dtype, consumer):
     text = b.build(b.convert(b.multiply(r, b.splat(0.5, r)), "bf16") if consumer else r)
     v = np.random.default_rng(18).standard_normal((R, N), dtype=np.float32).astype(configs.np_dtype(dtype))
     check_program(client, text, [v], f"column sum {dtype} {R}x{N}", f32_tol=1e-6)
+
+
+# several groups of heads (as many to a group as have 32 MiB of keys and values): a shorter last group, one head per group, and
+# one group as the limit, in both kernel forms, with every row of every head checked
+@pytest.mark.parametrize("BH,Sq,Sk,D,per_group", [(5, 300, 20000, 128, 3), (3, 200, 40000, 128, 1), (7, 257, 40000, 64, 3), (2, 300, 32768, 128, 2)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("form", ["tile", "persistent"])
+def test_attention_groups_of_heads(monkeypatch, BH, Sq, Sk, D, per_group, causal, form):
+    import ctypes as C
+
+    import torch
+
+    from ryft_b200 import kernels
+
+    class Args(C.Structure):
+        _fields_ = [("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("o", C.c_void_p), ("BH", C.c_int64), ("Sq", C.c_int64), ("Sk", C.c_int64), ("D", C.c_int64),
+                    ("scale", C.c_float), ("causal", C.c_int)]
+
+    assert max(1, min(BH, (32 << 20) // (Sk * D * 4))) == per_group
+    lib = kernels.load()
+    monkeypatch.setenv("B2X_ATTENTION_KERNEL", form)
+    g = torch.Generator(device="cuda").manual_seed(11)
+    q, k, v = (torch.randn((BH, n, D), generator=g, device="cuda").bfloat16() for n in (Sq, Sk, Sk))
+    o = torch.full((BH, Sq, D), float("nan"), device="cuda", dtype=torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a = Args(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), BH, Sq, Sk, D, D ** -0.5, int(causal))
+    lib.b2x_launch_attention.argtypes = [C.POINTER(Args), C.c_void_p, C.c_void_p]
+    assert lib.b2x_launch_attention(C.byref(a), status.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert status.item() == 0
+    for h in range(BH):
+        s = (q[h].double() @ k[h].double().T) * D ** -0.5
+        if causal:
+            s.masked_fill_(torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+        w = torch.softmax(s, dim=1)
+        want = w @ v[h].double()
+        # one rounding of the weights and one of the result to bf16, as above; the row sums are exact to 2^-20 or so
+        bound = 2 ** -8 * (w @ v[h].double().abs()) + 2 ** -7 * want.abs() + 1e-6
+        assert ((o[h].double() - want).abs() <= bound).all(), (h, (o[h].double() - want).abs().max().item())
+
+
+# the threefold split of f32 operands for a single product over 3 K: [hi | hi | lo] and [hi | lo | hi], bit for bit
+@pytest.mark.parametrize("B,M,N,K,lc,rc", [(1, 3, 5, 7, 1, 0), (2, 33, 130, 128, 0, 1), (1, 70, 129, 300, 1, 1), (3, 128, 32, 33, 0, 0)])
+def test_threefold_split(B, M, N, K, lc, rc):
+    import ctypes as C
+
+    import torch
+
+    from ryft_b200 import kernels
+
+    class Args(C.Structure):
+        _fields_ = [("a", C.c_void_p), ("b", C.c_void_p), ("elem", C.c_uint8)] + [(n, C.c_int64) for n in (
+            "batch", "M", "N", "K", "a_batch_stride", "a_row_stride", "a_k_stride", "b_batch_stride", "b_row_stride", "b_k_stride")]
+
+    lib = kernels.load()
+    r = np.random.default_rng(15)
+    a, b = r.standard_normal((B, M, K), dtype=np.float32), r.standard_normal((B, N, K), dtype=np.float32)
+    da, db = (torch.from_numpy(np.ascontiguousarray(x if c else x.swapaxes(1, 2))).cuda() for x, c in ((a, lc), (b, rc)))
+    sa, sb = (torch.full((B, rows, 3 * K), float("nan"), device="cuda") for rows in (M, N))
+    args = Args(da.data_ptr(), db.data_ptr(), kernels.EL_F32, B, M, N, K, M * K, K if lc else 1, 1 if lc else M, N * K, K if rc else 1, 1 if rc else N)
+    lib.b2x_launch_split_f32.argtypes = [C.POINTER(Args), C.c_void_p, C.c_void_p, C.c_void_p]
+    assert lib.b2x_launch_split_f32(C.byref(args), sa.data_ptr(), sb.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+    def cut(x):
+        return (x.view(np.uint32) & np.uint32(0xffffe000)).view(np.float32)
+    for got, x, order in ((sa, a, (0, 0, 1)), (sb, b, (0, 1, 0))):
+        halves = (cut(x), cut(x - cut(x)))
+        assert np.array_equal(got.cpu().numpy(), np.concatenate([halves[i] for i in order], axis=2))
+
+
+# a row softmax between other kernels: its operand made by a product and an elementwise step, or by a reduction; its result read
+# by a product
+@pytest.mark.parametrize("B,S,D", [(3, 70, 40), (2, 136, 64)])
+def test_row_softmax_between_products(client, B, S, D):
+    import ryft_b200
+    b = Builder()
+    x = b.arg([B, S, D], "f32"); y = b.arg([B, S, D], "f32")
+    s = b.dot_general(x, y, ([0], [0]), ([2], [2]))
+    s = b.multiply(s, b.splat(0.125, s))
+    m = b.reduce(s, b.constant(float("-inf"), [], "f32"), "maximum", [2])
+    e = b.exponential(b.subtract(s, b.broadcast_in_dim(m, [0, 1], [B, S, S])))
+    l = b.reduce(e, b.constant(0.0, [], "f32"), "add", [2])
+    q = b.divide(e, b.broadcast_in_dim(l, [0, 1], [B, S, S]))
+    text = b.build(b.dot_general(q, y, ([0], [0]), ([2], [1])))
+    assert "softmax softmax" in ryft_b200.plan_dump(text)
+    r = np.random.default_rng(16)
+    # a difference of 1e-6 in the scores (f32 sums over D) is one of 1e-6 in the weights
+    check_program(client, text, [r.standard_normal((B, S, D), dtype=np.float32) for _ in range(2)], f"attention in f32 {B}x{S}x{D}", f32_tol=5e-6)
+
+
+def test_row_softmax_of_a_reduction(client):
+    import ryft_b200
+    shape = [37, 50, 130]
+    b = Builder()
+    x = b.arg(shape, "f32")
+    y = b.reduce(x, b.constant(0.0, [], "f32"), "add", [1])
+    m = b.reduce(y, b.constant(float("-inf"), [], "f32"), "maximum", [1])
+    e = b.exponential(b.subtract(y, b.broadcast_in_dim(m, [0], [37, 130])))
+    s = b.reduce(e, b.constant(0.0, [], "f32"), "add", [1])
+    text = b.build(b.divide(e, b.broadcast_in_dim(s, [0], [37, 130])))
+    assert "softmax softmax" in ryft_b200.plan_dump(text)
+    # the sums of 50 normals (up to 30) round with 2^-24 of themselves a few times: as much in the exponentials
+    check_program(client, text, [np.random.default_rng(17).standard_normal(shape, dtype=np.float32)], "softmax of a reduction", f32_tol=1e-5)
+
+
+# kernels that start early reuse the blocks of one arena, execution after execution and on other arguments each time: what one
+# reads is what the kernels in front of it have written
+def test_back_to_back_executions_reuse_one_arena(client):
+    from ryft_b200 import pjrt
+    n = 160
+    b = Builder()
+    x = b.arg([n, n], "f32"); w = b.arg([n, n], "bf16")
+    y = x
+    for _ in range(4):
+        h = b.dot_general(b.convert(y, "bf16"), w, ([], []), ([1], [0]), out_dtype="f32")
+        t = b.reduce(b.multiply(h, h), b.constant(0.0, [], "f32"), "add", [0])
+        y = b.tanh(b.subtract(h, b.broadcast_in_dim(b.multiply(t, b.splat(1.0 / n, t)), [1], [n, n])))
+    exe = client.compile(pjrt.Program.mlir(b.build(y)))
+    r = np.random.default_rng(19)
+    wb = client.buffer((r.standard_normal((n, n), dtype=np.float32) * np.float32(n ** -0.5)).astype(BF16))
+    xs = [client.buffer(r.standard_normal((n, n), dtype=np.float32)) for _ in range(3)]
+    alone = []
+    for xb in xs:
+        out = exe.execute([pjrt.ExecutionDeviceInputs([xb, wb])])[0]
+        out.done.await_()
+        alone.append(out.outputs[0].to_numpy())
+    queued = [exe.execute([pjrt.ExecutionDeviceInputs([xs[i % 3], wb])])[0] for i in range(60)]
+    for i, out in enumerate(queued):
+        assert np.array_equal(out.outputs[0].to_numpy(), alone[i % 3]), i
+
+
+# two executables on two threads read one view; the view goes away while they are still queued
+def test_view_outlives_the_executions_of_two_threads(client):
+    import threading
+
+    import torch
+
+    from ryft_b200 import pjrt
+
+    def program(factor):
+        b = Builder()
+        x = b.arg([1 << 20], "f32")
+        y = x
+        for _ in range(20):
+            y = b.add(b.multiply(y, b.splat(0.5, y)), b.splat(factor, y))
+        return b.build(y)
+    exes = [client.compile(pjrt.Program.mlir(program(f))) for f in (0.25, 0.75)]
+    for _ in range(10):
+        t = torch.ones(1 << 20, device="cuda")
+        torch.cuda.synchronize()
+        view = client.view_of_device_buffer(t.data_ptr(), pjrt.BufferType.F32, [1 << 20], keep=t)
+        results = [[], []]
+
+        def work(i):
+            for _ in range(20):
+                results[i].append(exes[i].execute([pjrt.ExecutionDeviceInputs([view])])[0])
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+        for th in threads:
+            th.start()
+        for th in threads:
+            th.join()
+        del view                                  # waits for every reader
+        t.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for i, f in enumerate((0.25, 0.75)):
+            want = np.float32(1.0)
+            for _ in range(20):
+                want = np.float32(want * np.float32(0.5)) + np.float32(f)
+            for out in results[i]:
+                assert (out.outputs[0].to_numpy() == want).all()
