@@ -416,7 +416,7 @@ static int direct_kind(const B2xVmProgram& P, const ReduceKArgs& K, int vec) {
 // in shared memory, the CTAs of the cluster through distributed shared memory, always in the same order.
 // HBM-bound; what decides is how many bytes are in flight, i.e. how many CTAs there are.  [8192, 4096] f32 -> [4096]:
 // 3557 us with one CTA per 2048 columns and row split (8 CTAs, one interpreted row in flight per thread) and a second
-// launch for the four splits; 64 column blocks x 8 CTAs with eight 16-byte loads in flight per thread: 27.0 us (5.0 TB/s) on the device.
+// launch for the four splits; 64 column blocks x 8 CTAs with eight 16-byte loads in flight per thread: 25.6 us (5.2 TB/s) on the device.
 // DIRECT: the prologue is the dense tensor itself, f32 (4) or bf16 (2), and the loop is plain loads and arithmetic
 // (direct_cols); 0: the prologue program.  MC: see red_combine_t.  The vector forms are held to the 64 registers of four CTAs per
 // SM: left alone, the compiler takes 72 for bf16 ([8192, 4096] 19.4 us, 13.9 so) and spills in the f32 loop (27.1 us, 25.6 so).

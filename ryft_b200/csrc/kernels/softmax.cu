@@ -3,13 +3,14 @@
 // The planner recognises the chain reduce max -> subtract -> exponential -> reduce add -> divide over the last dimension
 // (crates/ryft-mlir/src/dialects/stable_hlo/operations/functional.rs:188-219 and the elementwise builders) and replaces
 // its four passes over memory with this one: a row is read once, kept in registers between the maximum, the exponentials
-// and the quotient, and written once.  The arithmetic is the chain's own (expf, IEEE division, f32 sums), so infinities
+// and the quotient, and written once.  The operations are the chain's own (expf, IEEE division, f32 sums; the terms of a sum
+// are added in another order, with an error against 64 bits that is no larger at any width), so infinities
 // and NaN go the same way: a NaN or +inf score, or a row of -inf only, makes the row NaN.
 //
 // HBM-bound: 4 bytes read and the result's bytes written per element.  A row belongs to a warp up to 1024 elements (two
 // shuffle reductions, no barrier) and to a CTA of 256 or 512 threads above; E elements per thread cover the row exactly
 // once, so E is the smallest power of two that does.  [8192, 4096] f32: 424 us in four passes, two of them interpreted
-// (805 MB); 45 us in one (5.95 TB/s). [1387, 151]: 38.9 us in four launches, 4.1 in one.
+// (805 MB); 43.6 us in one (6.15 TB/s). [1387, 151]: 38.9 us in four launches, 4.1 in one.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
