@@ -190,22 +190,16 @@ static __device__ __noinline__ void tc_settle(const float* a, const float* b, in
         const int i = __ffs(todo) - 1;
         const float* x = a + i * pitch;
         const float* y = b + (col + j) * pitch;
-        bool nan = false, pos = false, neg = false;      // of the whole row, after each round of 256 products
-        for (int64_t k0 = 0; k0 < K && !nan && !(pos && neg); k0 += 256) {
-#pragma unroll
-          for (int u = 0; u < 8; u++) {
-            const int64_t k = k0 + u * 32 + lane;
-            if (k < K) {
-              const float t = (ld_global(x + k) + ld_global(x + lo_off + k)) * (ld_global(y + k) + ld_global(y + lo_off + k));
-              nan |= t != t;
-              pos |= t == CUDART_INF_F;
-              neg |= t == -CUDART_INF_F;
-            }
-          }
-          nan = __any_sync(0xffffffffu, nan);
-          pos = __any_sync(0xffffffffu, pos);
-          neg = __any_sync(0xffffffffu, neg);
+        bool nan = false, pos = false, neg = false;
+        for (int64_t k = lane; k < K; k += 32) {
+          const float t = (ld_global(x + k) + ld_global(x + lo_off + k)) * (ld_global(y + k) + ld_global(y + lo_off + k));
+          nan |= t != t;
+          pos |= t == CUDART_INF_F;
+          neg |= t == -CUDART_INF_F;
         }
+        nan = __any_sync(0xffffffffu, nan);
+        pos = __any_sync(0xffffffffu, pos);
+        neg = __any_sync(0xffffffffu, neg);
         if (lane == i && !nan && pos != neg) c[j] = __float_as_uint(pos ? CUDART_INF_F : -CUDART_INF_F);
       }
     }
